@@ -93,7 +93,8 @@ def _load() -> C.CDLL:
             f"{LIB_PATH} is missing: build it with `python -m cachalot_b200.build` "
             "(needs nvcc; there is no CPU or PyTorch fallback for these kernels)"
         )
-    lib = C.CDLL(str(LIB_PATH))
+    # an override goes into the global scope, where the native call path (_host.so) finds it before its own copy
+    lib = C.CDLL(str(LIB_PATH), mode=C.RTLD_GLOBAL if "CACHALOT_B200_LIB" in os.environ else C.DEFAULT_MODE)
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError if the symbol is not exported
         fn.restype, fn.argtypes = res, args

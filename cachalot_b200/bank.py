@@ -135,6 +135,11 @@ class SlabBank:
         return int(self.desc.fp4_scale_centre)
 
     @property
+    def default_numerics(self) -> int:
+        """Rounding points of the bank's decode op: fp32 between the projections (FP4), bf16 (affine)."""
+        return _lib.NUMERICS_F32 if self.fmt.kind == "fp4" else _lib.NUMERICS_BF16
+
+    @property
     def desc_ptr(self):
         return C.byref(self.desc)
 

@@ -1,8 +1,9 @@
-"""In-tree build of the CUDA library for sm_100a.
+"""In-tree build of the CUDA library for sm_100a and of the native call path.
 
 `python -m cachalot_b200.build` (or `build()` from Python) compiles every `csrc/*.cu` with
-nvcc into `cachalot_b200/libcachalot_b200.so`.  nvcc cross-compiles without a GPU.  The
-library is rebuilt only when a source or header is newer than it.
+nvcc into `cachalot_b200/libcachalot_b200.so` (nvcc cross-compiles without a GPU) and
+`csrc/host/host.cpp` with the C++ compiler into the extension module `cachalot_b200/_host.so`.
+Each is rebuilt only when a source or header is newer than it.
 """
 from __future__ import annotations
 
@@ -10,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -17,6 +19,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = Path(os.environ.get("CACHALOT_B200_LIB", PKG / "libcachalot_b200.so"))
 OBJ_DIR = PKG / "csrc" / "build"
+HOST_SRC = CSRC / "host" / "host.cpp"
+HOST_LIB = PKG / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -48,9 +52,38 @@ def needs_build() -> bool:
     return any(p.stat().st_mtime > t for p in _deps())
 
 
+def build_host(force: bool = False) -> Path:
+    """The extension module that ops.py calls (it links the CUDA library beside it by its own location)."""
+    deps = [HOST_SRC, PKG.parent / "include" / "cachalot_b200.h"]
+    if not force and HOST_LIB.exists() and all(p.stat().st_mtime <= HOST_LIB.stat().st_mtime for p in deps):
+        return HOST_LIB
+    from torch.utils import cpp_extension
+
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(_torch_cxx11_abi())}", "-I" + sysconfig.get_paths()["include"],
+           "-I" + str(Path(_nvcc()).resolve().parents[1] / "include"), *("-isystem" + p for p in cpp_extension.include_paths()),
+           str(HOST_SRC), "-o", str(HOST_LIB), *("-L" + p for p in cpp_extension.library_paths()), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
+           "-lc10_cuda", "-lc10", "-L" + str(LIB.parent), "-l:" + LIB.name, "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"host module failed:\n{res.stdout}\n{res.stderr}")
+    return HOST_LIB
+
+
+def _torch_cxx11_abi() -> bool:
+    import torch
+
+    return torch._C._GLIBCXX_USE_CXX11_ABI
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    if not force and not needs_build():
-        return LIB
+    if force or needs_build():
+        _build_cuda(verbose)
+    build_host(force)
+    return LIB
+
+
+def _build_cuda(verbose: bool = False) -> Path:
     nvcc = _nvcc()
     OBJ_DIR.mkdir(exist_ok=True)
     extra = ["-Xptxas", "-v"] if verbose else []

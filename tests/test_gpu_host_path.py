@@ -1,0 +1,96 @@
+"""The native call path of the operators gives what their general form gives: the same kernels on the same bytes, so the
+same bits.  A float32 or strided activation (bf16 values either way) is what the native path hands over to the general one."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def bank():
+    import cachalot_b200 as cb
+
+    b = cb.SlabBank(cb.FP4_FORMAT, 512, 384, 16, layers=2, n_experts=8)
+    b.fill_random(torch.Generator(device="cuda").manual_seed(1))
+    return b
+
+
+def _fp8(n, k, rule, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = (torch.randn((n, k), device="cuda", generator=g) * 64).to(torch.float8_e4m3fn).view(torch.uint8)
+    if rule == "e8m0":
+        return w, torch.randint(112, 116, (-(-n // 32), k // 32), device="cuda", generator=g).to(torch.uint8)
+    return w, torch.rand((-(-n // 128), k // 128), device="cuda", generator=g) * 1e-3
+
+
+def _x(*shape):
+    return torch.randn(shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("rule", ["e8m0", "f32"])
+@pytest.mark.parametrize("rows", [None, 1, 3])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_fp8_linear(rule, rows, dtype):
+    import cachalot_b200 as cb
+
+    x = _x(384) if rows is None else _x(rows, 384)
+    w, s = _fp8(200, 384, rule, 3)
+    assert torch.equal(cb.fp8_linear(x, w, s, out_dtype=dtype), cb.fp8_linear(x.float(), w, s, out_dtype=dtype))
+
+
+@pytest.mark.parametrize("rows", [None, 1, 9])
+def test_bf16_gemv(rows):
+    import cachalot_b200 as cb
+
+    x = _x(320) if rows is None else _x(rows, 320)
+    w = _x(77, 320)
+    assert torch.equal(cb.bf16_gemv_f32(x.float(), w), cb.bf16_gemv_f32(x, w))
+
+
+@pytest.mark.parametrize("rows", [1, 3, 9])
+def test_moe_forward(bank, rows):
+    import cachalot_b200 as cb
+
+    x = _x(rows, bank.hidden)
+    slots = torch.arange(rows * 4, device="cuda", dtype=torch.int32).reshape(rows, 4) % 16
+    w = torch.rand((rows, 4), device="cuda")
+    assert torch.equal(cb.moe_forward(x, slots, w, bank), cb.moe_forward(x.float(), slots.long(), w, bank))
+
+
+@pytest.mark.parametrize("want", [False, True])
+def test_layer_decode(bank, want):
+    import cachalot_b200 as cb
+
+    x, logits, bias = _x(bank.hidden), torch.randn(8, device="cuda"), torch.randn(8, device="cuda")
+    a = cb.moe_layer_decode(x, logits, bank, layer=1, topk=3, bias=bias, want_routing=want)
+    b = cb.moe_layer_decode(x.float(), logits, bank, layer=1, topk=3, bias=bias, want_routing=want)
+    for u, v in zip(a if want else [a], b if want else [b]):
+        assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("mx", [0, 1])
+def test_prefill(bank, mx):
+    import cachalot_b200 as cb
+
+    x, ids = _x(37, bank.hidden), torch.randint(0, 8, (37, 2), device="cuda", dtype=torch.int32)
+    w = torch.rand((37, 2), device="cuda")
+    a = cb.moe_prefill_grouped(x, ids, w, bank, layer=1, mxfp4_act=mx)
+    assert torch.equal(a, cb.moe_prefill_grouped(x.float(), ids, w, bank, layer=1, mxfp4_act=mx))
+
+
+@pytest.mark.parametrize("rule", ["e8m0", "f32"])
+@pytest.mark.parametrize("fused13", [False, True])
+def test_block(bank, rule, fused13):
+    import cachalot_b200 as cb
+
+    h, i = bank.hidden, 256
+    (w1, s1), (w3, s3), (w2, s2) = _fp8(i, h, rule, 4), _fp8(i, h, rule, 5), _fp8(h, i, rule, 6)
+    if fused13:
+        w1, s1, w3, s3 = torch.cat([w1, w3]), torch.cat([s1, s3]), None, None
+    x, gate, bias = _x(h), _x(8, h), torch.randn(8, device="cuda")
+    kw = dict(layer_id=1, gate_weight=gate, gate_bias=bias, expert_store=bank, shared_w1=w1, shared_w1_scales=s1, shared_w2=w2,
+              shared_w2_scales=s2, shared_w3=w3, shared_w3_scales=s3, topk=3)
+    (a, ra), (b, rb) = cb.moe_layer_forward(x, **kw), cb.moe_layer_forward(x.float(), **kw)
+    assert torch.equal(a, b) and torch.equal(ra.indices, rb.indices) and torch.equal(ra.weights, rb.weights) and torch.equal(ra.scores, rb.scores)
+    y = cb.shared_expert_forward_batched(_x(5, h), w1=w1, w1_scales=s1, w3=w3, w3_scales=s3, w2=w2, w2_scales=s2)
+    assert torch.equal(y, cb.shared_expert_forward_batched(_x(5, h).float(), w1=w1, w1_scales=s1, w3=w3, w3_scales=s3, w2=w2, w2_scales=s2))
