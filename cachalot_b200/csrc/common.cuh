@@ -39,6 +39,16 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 
 // ---- device helpers ---------------------------------------------------------------------
 
+// One lane of a converged warp.  Instructions that take their operands from uniform registers (tcgen05.mma, .cp and
+// .commit, TMA loads) belong under this predicate and not under `lane == 0`: only here does the compiler know that one
+// thread is active; under any other condition it wraps each of them in a loop over the active threads (measured:
+// 155 cycles per tcgen05.mma kind::f16 M=128 N=16..128 under `lane == 0`, 19 at N=16 and 64 at N=128 under elect).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.b32 %0, 1, 0, P;\n}" : "=r"(p));
+  return p != 0;
+}
+
 // 128-bit streaming load: weights are read exactly once, so keep them out of L1.
 __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
   uint4 v;

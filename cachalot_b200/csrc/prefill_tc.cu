@@ -262,7 +262,7 @@ grouped_mxf4_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
 
   if (warp == 0) {
     // ---- tile loads ------------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       // weights are read once: first out of L2; activation rows are re-read by every tile of the expert
       uint64_t pol_w, pol_x;
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
@@ -337,7 +337,7 @@ grouped_mxf4_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
     // ---- scale copies into TMEM and the MMAs -------------------------------------------------
     // One thread issues everything, so its own instruction count is on the critical path: all descriptors are
     // the stage's base descriptor plus a compile-time constant (addresses are in 16-byte units in the low bits).
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       long long item = 0;
