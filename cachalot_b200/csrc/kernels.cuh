@@ -85,7 +85,7 @@ int launch_prefill_rows(const BankView& v, const uint8_t* x_codes, const uint8_t
                         const int32_t* seg_offsets, const int32_t* seg_slot, int n_seg, long long rows, float limit, bool zero_absent,
                         void* workspace, __nv_bfloat16* y, int* status, cudaStream_t stream);
 size_t prefill_rows_workspace_bytes(int inter, long long rows, int n_seg);
-int launch_combine_rows(const __nv_bfloat16* y, const int32_t* inv, int tokens, int k, int hidden, float* out, cudaStream_t stream);
+int launch_combine_rows(const __nv_bfloat16* y, const int32_t* inv, int tokens, int k, int hidden, void* out, int out_dtype, cudaStream_t stream);
 bool prefill_tc_supported(const BankView& v);
 // decode batches through the same grouped kernels (FP4 bank, fp32 numerics), every distinct expert streamed once
 int launch_decode_tc(const BankView& v, const void* x_bf16, const int32_t* slots, const float* gate_w, int rows, int k, float limit,
@@ -98,5 +98,16 @@ int launch_prefill_exact(const BankView& v, const void* x_bf16, const int32_t* p
                          cudaStream_t stream);
 size_t decode_tc_workspace_bytes(int hidden, int inter, int rows, int k);
 bool decode_tc_supported(const BankView& v, int rows, int k);
+
+// Several tokens over the 2-bit bank (fp16 scales, the reference's bf16 rounding points) on the f16 tensor cores, every
+// distinct expert streamed once (grouped_f16.cu).
+bool f16_supported(const BankView& v);
+size_t decode_f16_workspace_bytes(const BankView& v, int rows, int k);
+int launch_decode_f16(const BankView& v, const void* x_bf16, const int32_t* slots, const float* gate_w, int rows, int k, float limit,
+                      void* workspace, void* out, int out_dtype, int* status, cudaStream_t stream);
+size_t prefill_f16_workspace_bytes(const BankView& v, int tokens, int k, int n_experts);
+int launch_prefill_f16(const BankView& v, const void* x_bf16, const int32_t* perm, const int32_t* offsets, const int32_t* slot_of_expert,
+                       const float* gate_w, int tokens, int k, int n_experts, float limit, void* workspace, float* out, int* status,
+                       cudaStream_t stream);
 
 }  // namespace cachalot

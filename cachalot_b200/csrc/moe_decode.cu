@@ -286,9 +286,20 @@ static int grouped_tc_min_rows() {  // CACHALOT_GROUPED_MIN_ROWS overrides the b
   return v;
 }
 #define GROUPED_TC_MIN_ROWS grouped_tc_min_rows()
+// 2-bit bank with fp16 scales, reference rounding points: the grouped f16 kernels pay per distinct expert (about 11 us at
+// 4096 x 2880: unpacking its codes), the per-token kernel per routed row (3.8 us), so the former take the call when the
+// rows are at least three times the experts there can be.
+static bool grouped_f16_pays(long long routed_rows, long long n_experts) { return routed_rows >= 3 * n_experts; }
 
-extern "C" size_t cachalot_moe_decode_workspace_bytes(const cachalot_bank_desc* desc, int rows, int k) {
-  if (!desc || rows <= 0 || k <= 0) return 0;
+// the descriptor's fields that f16_supported() and its scratch sizes look at
+static BankView shape_view(const cachalot_bank_desc* d) {
+  BankView v = {};
+  v.format = d->format, v.bits = d->bits, v.group = d->group, v.scale_dtype = d->scale_dtype, v.hidden = d->hidden, v.inter = d->inter;
+  return v;
+}
+
+// what moe_decode cannot do without; with less than cachalot_moe_decode_workspace_bytes a 2-bit bank goes token by token
+static size_t decode_min_workspace(const cachalot_bank_desc* desc, int rows, int k) {
   const size_t a = decode_mma_workspace_bytes(desc->hidden, desc->inter, rows, k);  // >= the simple kernels' rows*k*inter floats
   const size_t b = decode_fused_workspace_bytes(desc->hidden, desc->inter, rows, k);
   size_t c = 0;
@@ -296,6 +307,14 @@ extern "C" size_t cachalot_moe_decode_workspace_bytes(const cachalot_bank_desc* 
     c = decode_tc_workspace_bytes(desc->hidden, desc->inter, rows, k);
   const size_t m = a > b ? a : b;
   return m > c ? m : c;
+}
+
+extern "C" size_t cachalot_moe_decode_workspace_bytes(const cachalot_bank_desc* desc, int rows, int k) {
+  if (!desc || rows <= 0 || k <= 0) return 0;
+  const size_t m = decode_min_workspace(desc, rows, k);
+  const BankView v = shape_view(desc);
+  const size_t f = f16_supported(v) && grouped_f16_pays((long long)rows * k, desc->n_slots) && k <= 64 ? decode_f16_workspace_bytes(v, rows, k) : 0;
+  return m > f ? m : f;
 }
 
 extern "C" int cachalot_moe_decode(const void* bank, const cachalot_bank_desc* desc, const void* x_bf16,
@@ -312,7 +331,7 @@ extern "C" int cachalot_moe_decode(const void* bank, const cachalot_bank_desc* d
     return fail(CACHALOT_EINVAL, "moe_decode: unknown numerics %d", numerics);
   if (out_dtype != CACHALOT_F32 && out_dtype != CACHALOT_BF16) return fail(CACHALOT_EINVAL, "moe_decode: out dtype must be f32 or bf16");
   if (rows == 0) return CACHALOT_OK;
-  size_t need = cachalot_moe_decode_workspace_bytes(desc, rows, k);
+  const size_t need = decode_min_workspace(desc, rows, k);
   if (!workspace || workspace_bytes < need) return fail(CACHALOT_ESCRATCH, "moe_decode: workspace %zu < %zu bytes", workspace_bytes, need);
   if (!aligned(workspace, 256) || !aligned(x_bf16, 16) || !aligned(out, 4)) return fail(CACHALOT_EALIGN, "moe_decode: workspace needs 256-byte, x 16-byte alignment");
   const bool fused_ok = !(numerics & (CACHALOT_DECODE_SIMPLE | CACHALOT_DECODE_UNFUSED | CACHALOT_DECODE_ONLY_GATE_UP | CACHALOT_DECODE_ONLY_DOWN));
@@ -322,12 +341,16 @@ extern "C" int cachalot_moe_decode(const void* bank, const cachalot_bank_desc* d
       ((numerics & 0xff) == CACHALOT_NUMERICS_F32 || (numerics & 0xff) == CACHALOT_NUMERICS_BF16))
     return launch_decode_tc(v, x_bf16, slots, gate_w, rows, k, swiglu_limit, workspace, out, out_dtype, status, (cudaStream_t)stream,
                             (numerics & 0xff) == CACHALOT_NUMERICS_BF16);
+  if (fused_ok && f16_supported(v) && grouped_f16_pays((long long)rows * k, v.n_slots) && (numerics & 0xff) == CACHALOT_NUMERICS_BF16 &&
+      workspace_bytes >= decode_f16_workspace_bytes(v, rows, k))
+    return launch_decode_f16(v, x_bf16, slots, gate_w, rows, k, swiglu_limit, workspace, out, out_dtype, status, (cudaStream_t)stream);
   // Up to 64 tokens: one single-launch kernel per token, back to back.  Tokens share few experts at these sizes (384
   // routed rows touch about 244 of 384 experts), so grouping rows by expert saves less than the per-token kernel
-  // gains by streaming its experts about twice as fast as the grouped kernels (measured: FP4 bank, 8 tokens 0.29 ms
-  // per layer against 0.64 ms, 64 tokens 2.24 ms against 2.98 ms).
-  // The 2-bit bank has no grouped kernel that beats the per-token one at any row count (measured up to 4096 tokens:
-  // 21-25 us per token against ~100 us per token on the grouped and the one-warp-per-output kernels).
+  // gains by streaming its experts about twice as fast as the grouped mma.sync kernels (measured: FP4 bank, 8 tokens
+  // 0.29 ms per layer against 0.64 ms, 64 tokens 2.24 ms against 2.98 ms).
+  // The 2-bit bank where the f16 kernels do not apply (bf16 scales, fp32 numerics): the per-token kernel at any row
+  // count (measured up to 4096 tokens: 21-25 us per token against ~100 us per token on the grouped mma.sync and the
+  // one-warp-per-output kernels).
   if (fused_ok && (rows <= FUSED_PER_TOKEN_MAX_ROWS || v.format == CACHALOT_BANK_AFFINE) && decode_fused_supported(v, 1, k)) {
     const size_t out_row = (size_t)v.hidden * (out_dtype == CACHALOT_BF16 ? 2 : 4);
     for (int r = 0; r < rows; ++r) {
@@ -461,6 +484,11 @@ extern "C" size_t cachalot_moe_prefill_workspace_bytes(const cachalot_bank_desc*
   size_t b = align_up(rows * desc->inter * sizeof(float), 256);   // hidden
   b += align_up(rows * sizeof(int32_t), 256);                     // slot per routed row
   if (mxfp4_act) b += align_up((size_t)tokens * desc->hidden * 2, 256);  // MXFP4-rounded x as bf16
+  const BankView v = shape_view(desc);
+  if (!mxfp4_act && f16_supported(v) && rows <= 65535) {  // the expert count is not known here
+    const size_t f = prefill_f16_workspace_bytes(v, tokens, k, 8192);
+    if (f > b) b = f;
+  }
   if (mxfp4_act == 1 && desc->format == CACHALOT_BANK_FP4) {
     // experts without rows get no unit, so the unit list is bounded by the rows whatever the number of experts is
     const size_t tc = prefill_tc_workspace_bytes(desc->hidden, desc->inter, tokens, k, tokens * k);
@@ -495,6 +523,8 @@ extern "C" int cachalot_moe_prefill(const void* bank, const cachalot_bank_desc* 
   if (tc)
     return launch_prefill_tc(v, x_bf16, perm, offsets, slot_of_expert, gate_w, tokens, k, n_experts, swiglu_limit, workspace, out,
                              status, s);
+  if (!mxfp4_act && f16_supported(v) && n_experts <= 8192 && grouped_f16_pays(rows, n_experts))
+    return launch_prefill_f16(v, x_bf16, perm, offsets, slot_of_expert, gate_w, tokens, k, n_experts, swiglu_limit, workspace, out, status, s);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   float* hidden = reinterpret_cast<float*>(ws);
   ws += align_up(rows * desc->inter * sizeof(float), 256);
@@ -513,8 +543,8 @@ extern "C" int cachalot_moe_prefill(const void* bank, const cachalot_bank_desc* 
   rc = check_launch("moe_prefill slots");
   if (rc) return rc;
   const int num = mxfp4_act ? CACHALOT_NUMERICS_BF16_H32 : CACHALOT_NUMERICS_BF16;
-  // bf16 activations where no tensor-core path exists (the 2-bit bank): the single-launch kernel, token by token - a
-  // quarter of the time of the one-warp-per-output kernels (86 ms against 400 ms for 4096 tokens at 4096 x 2880)
+  // bf16 activations where the f16 kernels do not apply (a 2-bit bank with bf16 scales): the single-launch kernel, token
+  // by token - a quarter of the time of the one-warp-per-output kernels (86 ms against 400 ms for 4096 tokens at 4096 x 2880)
   if (!mxfp4_act && decode_fused_supported(v, 1, k)) {
     for (int r = 0; r < tokens; ++r) {
       rc = launch_decode_fused(v, static_cast<const __nv_bfloat16*>(x_in) + (size_t)r * v.hidden, slots + (size_t)r * k, gate_w + (size_t)r * k, 1,
@@ -558,7 +588,7 @@ extern "C" int cachalot_moe_combine_rows(const void* y_bf16, const int32_t* inv,
                                          cachalot_stream_t stream) {
   if (!y_bf16 || !inv || !out) return fail(CACHALOT_EINVAL, "moe_combine_rows: null pointer");
   if (tokens < 0 || k <= 0 || hidden <= 0 || hidden % 2) return fail(CACHALOT_EINVAL, "moe_combine_rows: bad shape");
-  return launch_combine_rows(static_cast<const __nv_bfloat16*>(y_bf16), inv, tokens, k, hidden, out, (cudaStream_t)stream);
+  return launch_combine_rows(static_cast<const __nv_bfloat16*>(y_bf16), inv, tokens, k, hidden, out, CACHALOT_F32, (cudaStream_t)stream);
 }
 
 // ---- decode with built-in scratch (no allocation anywhere) ------------------------------------
@@ -587,7 +617,7 @@ extern "C" int cachalot_moe_decode_static(const void* bank, const cachalot_bank_
                                           cachalot_stream_t stream) {
   if (!desc) return fail(CACHALOT_EINVAL, "moe_decode_static: null bank descriptor");
   if (rows > 0 && k > 0) {
-    const size_t need = cachalot_moe_decode_workspace_bytes(desc, rows, k);
+    const size_t need = decode_min_workspace(desc, rows, k);
     if (need > STATIC_SCRATCH_BYTES)
       return fail(CACHALOT_ESCRATCH,
                   "moe_decode_static: rows=%d k=%d needs %zu bytes of scratch but the built-in scratch holds %zu; "

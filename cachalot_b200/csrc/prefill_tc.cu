@@ -20,9 +20,7 @@
 //
 // Every wait is bounded: when one gives up the CTA raises CACHALOT_STATUS_WAIT_EXPIRED, all roles leave
 // their loops, TMEM is released and the kernel returns.
-#include <cuda.h>
-
-#include "kernels.cuh"
+#include "tensor_core.cuh"
 
 namespace cachalot {
 namespace {
@@ -36,79 +34,7 @@ constexpr int SF_TILE = 1024;    // 128 rows x 8 scale bytes, as two 512-byte gr
 constexpr int NTHREADS = 448;
 constexpr int TMEM_COLS = 512;
 constexpr int SF_COL = 2 * 2 * NTMAX;  // scale columns start behind the (up to) four accumulators
-constexpr uint32_t WAIT_LIMIT = 1u << 20;
 
-
-struct Unit {
-  int32_t slot, row_start, ntok, pad;
-};
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* b, int n) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// false when the wait gave up (it sets *abort) or another role already had
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort) {
-  for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-    if (mbar_try(b, parity)) return true;
-    if ((i & 63u) == 63u && *abort) return false;
-  }
-  *abort = 1;
-  return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar, uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::
-          "r"(smem_u32(dst)),
-      "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar)), "l"(policy)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar,
-                                            uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], "
-      "%6;" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)), "l"(policy)
-      : "memory");
-}
-
-// contiguous bytes -> shared memory (both 16-byte aligned, size a multiple of 16), completion on an mbarrier
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src),
-               "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-// pulls one weight tile into L2 ahead of its load
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
-
-// shared-memory matrix descriptors (address and offsets in 16-byte units, descriptor version 1)
-// operand tile: rows of 128 bytes, 128-byte swizzle, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// scale group: 32 rows of 16 bytes, no swizzle, 8-row groups 128 bytes apart
-__device__ __forceinline__ uint64_t desc_sf(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (8ull << 32) | (1ull << 46);
-}
 // instruction descriptor of kind::mxf4: E2M1 x E2M1, both K-major, E8M0 scales, M = 128, N = n
 __device__ __forceinline__ uint32_t idesc_mxf4(int n) {
   return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | ((uint32_t)(BM >> 4) << 24);
@@ -125,21 +51,6 @@ __device__ __forceinline__ void tc_mma(uint32_t tacc, uint64_t da, uint64_t db, 
       "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
 struct GemmArgs {
   const uint8_t* bank;        // slot records
   long long record_bytes;
@@ -630,7 +541,7 @@ grouped_mxf4_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
 // one CTA per expert: inverse permutation and source token of every grouped row of a present expert
 __global__ void plan_rows_kernel(const int32_t* __restrict__ perm, const int32_t* __restrict__ offsets,
                                  const int32_t* __restrict__ slot_of_expert, int n_slots, int k, const float* __restrict__ gate_w,
-                                 int32_t* __restrict__ inv, int32_t* __restrict__ src_token, float* __restrict__ row_w,
+                                 bool check_w, int32_t* __restrict__ inv, int32_t* __restrict__ src_token, float* __restrict__ row_w,
                                  int* __restrict__ status) {
   const int e = blockIdx.x;
   const int s = slot_of_expert ? slot_of_expert[e] : e;
@@ -640,13 +551,14 @@ __global__ void plan_rows_kernel(const int32_t* __restrict__ perm, const int32_t
     const int r = perm[p];
     src_token[p] = r / k;
     row_w[p] = gate_w[r];
+    if (check_w && status && !(fabsf(gate_w[r]) <= 3.0e38f)) atomicOr(status, CACHALOT_STATUS_BAD_WEIGHT);
     if (present) inv[r] = p;
   }
 }
 
-// single CTA: units of up to NTMAX rows per present expert, experts ascending
+// single CTA: units of up to max_rows rows per present expert, experts ascending
 __global__ void plan_units_kernel(const int32_t* __restrict__ offsets, const int32_t* __restrict__ slot_of_expert, int n_experts,
-                                  int n_slots, Unit* __restrict__ units, int32_t* __restrict__ n_units) {
+                                  int n_slots, int max_rows, Unit* __restrict__ units, int32_t* __restrict__ n_units) {
   extern __shared__ int32_t sh[];  // [blockDim.x] unit counts of each thread's span
   const int t = threadIdx.x, nt = blockDim.x;
   const int per = (n_experts + nt - 1) / nt;
@@ -654,7 +566,7 @@ __global__ void plan_units_kernel(const int32_t* __restrict__ offsets, const int
   auto units_of = [&](int e) {
     const int s = slot_of_expert ? slot_of_expert[e] : e;
     if (s < 0 || s >= n_slots) return 0;
-    return (offsets[e + 1] - offsets[e] + NTMAX - 1) / NTMAX;
+    return (offsets[e + 1] - offsets[e] + max_rows - 1) / max_rows;
   };
   int sum = 0;
   for (int e = lo; e < hi; ++e) sum += units_of(e);
@@ -678,8 +590,8 @@ __global__ void plan_units_kernel(const int32_t* __restrict__ offsets, const int
     for (int i = 0; i < nu; ++i) {
       Unit u;
       u.slot = s;
-      u.row_start = begin + i * NTMAX;
-      u.ntok = min(NTMAX, end - u.row_start);
+      u.row_start = begin + i * max_rows;
+      u.ntok = min(max_rows, end - u.row_start);
       u.pad = 0;
       units[at++] = u;
     }
@@ -698,8 +610,9 @@ __global__ void zero_absent_rows_kernel(const int32_t* __restrict__ offsets, con
 }
 
 // out[t, :] = sum over the token's route slots j = 0..k-1 (in that order) of its row of y
+template <typename OutT>
 __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ inv, int k, int hidden,
-                               float* __restrict__ out) {
+                               OutT* __restrict__ out) {
   const int t = blockIdx.x;
   for (int n = threadIdx.x * 2; n < hidden; n += blockDim.x * 2) {
     float a = 0.f, b = 0.f;
@@ -710,44 +623,16 @@ __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_
       a += __bfloat162float(v.x);
       b += __bfloat162float(v.y);
     }
-    out[(size_t)t * hidden + n] = a;
-    out[(size_t)t * hidden + n + 1] = b;
+    OutT* o = out + (size_t)t * hidden + n;
+    if constexpr (sizeof(OutT) == 2)
+      o[0] = __float2bfloat16_rn(a), o[1] = __float2bfloat16_rn(b);
+    else
+      o[0] = a, o[1] = b;
   }
 }
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
-// byte matrix [planes][rows][row_bytes] with the given pitches; box = {128 bytes, box_rows, 1}, 128-byte swizzle
-int make_map(CUtensorMap* m, const void* base, int row_bytes, long long row_pitch, int rows, long long plane_pitch, int planes,
-             int box_rows) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return fail(CACHALOT_ECUDA, "moe_prefill: cuTensorMapEncodeTiled is not available from this driver");
-  cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)rows, (cuuint64_t)planes};
-  cuuint64_t strides[2] = {(cuuint64_t)row_pitch, (cuuint64_t)plane_pitch};
-  cuuint32_t box[3] = {(cuuint32_t)BKB, (cuuint32_t)box_rows, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  const int rank = planes > 0 ? 3 : 2;
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, rank, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(CACHALOT_ECUDA, "moe_prefill: cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return CACHALOT_OK;
-}
 
 constexpr int KSUB = 2;
 constexpr int STAGES_GU = 4 / KSUB, STAGES_DN = 6 / KSUB;
@@ -814,10 +699,10 @@ Scratch carve(uint8_t* base, int hidden, int inter, size_t rows, int n_experts) 
 constexpr int DTERMS = 4;  // MXFP4 rows per routed row
 
 // single CTA: routed rows (token * k + route slot) ordered by bank slot, stable; runs of one slot become segments of
-// DTERMS rows per routed row.  seg_off i32 [R + 1] (in MXFP4 rows), seg_slot i32 [R] (-1 behind the last segment and
+// `mul` rows per routed row.  seg_off i32 [R + 1] (in those rows), seg_slot i32 [R] (-1 behind the last segment and
 // for rows whose slot is absent or out of range), inv i32 [R] (position of a routed row in the order, -1 if absent),
 // src_token i32 [R] and row_w f32 [R] in the order.
-__global__ void decode_plan_kernel(const int32_t* __restrict__ slots, const float* __restrict__ gate_w, int R, int k, int n_slots,
+__global__ void decode_plan_kernel(const int32_t* __restrict__ slots, const float* __restrict__ gate_w, int R, int k, int n_slots, int mul,
                                    int32_t* __restrict__ seg_off, int32_t* __restrict__ seg_slot, int32_t* __restrict__ inv,
                                    int32_t* __restrict__ src_token, float* __restrict__ row_w, int* __restrict__ status) {
   extern __shared__ int32_t sh[];  // [R] slot of every row, [R] slot by position
@@ -850,12 +735,12 @@ __global__ void decode_plan_kernel(const int32_t* __restrict__ slots, const floa
     int ng = 0;
     for (int i = 0; i < R; ++i)
       if (i == 0 || s_sorted[i] != s_sorted[i - 1]) {
-        seg_off[ng] = i * DTERMS;
+        seg_off[ng] = i * mul;
         seg_slot[ng] = s_sorted[i];
         ++ng;
       }
     for (int gidx = ng; gidx <= R; ++gidx) {
-      seg_off[gidx] = R * DTERMS;
+      seg_off[gidx] = R * mul;
       if (gidx < R) seg_slot[gidx] = -1;
     }
   }
@@ -954,6 +839,60 @@ DecodeScratch carve_decode(uint8_t* base, int hidden, int inter, size_t R, size_
 
 }  // namespace
 
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiledFn encode_fn() {
+  static EncodeTiledFn fn = nullptr;
+  if (!fn) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<EncodeTiledFn>(p);
+  }
+  return fn;
+}
+
+int make_map(CUtensorMap* m, const void* base, int row_bytes, long long row_pitch, int rows, long long plane_pitch, int planes,
+             int box_rows, int box_bytes) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(CACHALOT_ECUDA, "moe_prefill: cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)rows, (cuuint64_t)planes};
+  cuuint64_t strides[2] = {(cuuint64_t)row_pitch, (cuuint64_t)plane_pitch};
+  cuuint32_t box[3] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const int rank = planes > 0 ? 3 : 2;
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, rank, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(CACHALOT_ECUDA, "moe_prefill: cuTensorMapEncodeTiled failed (%d)", (int)r);
+  return CACHALOT_OK;
+}
+
+// Plans of the grouped kernels: rows of a decode batch ordered by slot (R <= PLAN_ROWS_MAX), or the grouping of a prefill
+// chunk; `mul` rows of the GEMM per routed row, units of up to `nt` of them.
+int launch_decode_plan(const PlanArrays& p, const int32_t* slots, const float* gate_w, int R, int k, int n_slots, int mul, int nt,
+                       int* status, cudaStream_t stream) {
+  const int threads = R < 1024 ? ((R + 31) / 32) * 32 : 1024;
+  decode_plan_kernel<<<1, threads, 2 * R * sizeof(int32_t), stream>>>(slots, gate_w, R, k, n_slots, mul, p.seg_off, p.seg_slot, p.inv,
+                                                                    p.src_token, p.row_w, status);
+  plan_units_kernel<<<1, 256, 256 * sizeof(int32_t), stream>>>(p.seg_off, p.seg_slot, R, n_slots, nt, p.units, p.n_units);
+  return check_launch("moe_decode (grouped) plan");
+}
+int launch_prefill_plan(const PlanArrays& p, const int32_t* perm, const int32_t* offsets, const int32_t* slot_of_expert,
+                        const float* gate_w, long long R, int k, int n_experts, int n_slots, int nt, bool check_w, int* status,
+                        cudaStream_t stream) {
+  cudaError_t e = cudaMemsetAsync(p.inv, 0xFF, R * 4, stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p.src_token, 0, R * 4, stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p.row_w, 0, R * 4, stream);
+  if (e != cudaSuccess) return fail(CACHALOT_ECUDA, "moe_prefill: %s", cudaGetErrorString(e));
+  plan_rows_kernel<<<n_experts, 128, 0, stream>>>(perm, offsets, slot_of_expert, n_slots, k, gate_w, check_w, p.inv, p.src_token, p.row_w,
+                                                 status);
+  plan_units_kernel<<<1, 256, 256 * sizeof(int32_t), stream>>>(offsets, slot_of_expert, n_experts, n_slots, nt, p.units, p.n_units);
+  return check_launch("moe_prefill plan");
+}
+
 bool decode_tc_supported(const BankView& v, int rows, int k) {
   return prefill_tc_supported(v) && rows >= 1 && (long long)rows * k <= 1024;
 }
@@ -964,15 +903,15 @@ size_t decode_tc_workspace_bytes(int hidden, int inter, int rows, int k) { retur
 static int run_terms4(const BankView& v, const DecodeScratch& s, const int32_t* seg_off, const int32_t* seg_slot, int n_seg, long long Q,
                       float limit, bool round_bf16, int* status, cudaStream_t stream) {
   const int H = v.hidden, I = v.inter;
-  plan_units_kernel<<<1, 256, 256 * sizeof(int32_t), stream>>>(seg_off, seg_slot, n_seg, v.n_slots, s.units, s.n_units);
+  plan_units_kernel<<<1, 256, 256 * sizeof(int32_t), stream>>>(seg_off, seg_slot, n_seg, v.n_slots, NTMAX, s.units, s.n_units);
   int rc;
   if ((rc = check_launch("moe (grouped, exact activations) plan"))) return rc;
   CUtensorMap m_w1, m_w3, m_w2, m_x, m_h;
-  if ((rc = make_map(&m_w1, v.base + v.off[0], H / 2, H / 2, I, v.record_bytes, v.n_slots, BM))) return rc;
-  if ((rc = make_map(&m_w3, v.base + v.off[4], H / 2, H / 2, I, v.record_bytes, v.n_slots, BM))) return rc;
-  if ((rc = make_map(&m_w2, v.base + v.off[2], I / 2, I / 2, H, v.record_bytes, v.n_slots, BM))) return rc;
-  if ((rc = make_map(&m_x, s.x_codes, H / 2, H / 2, (int)Q, 0, 0, NTMAX))) return rc;
-  if ((rc = make_map(&m_h, s.h_codes, I / 2, I / 2, (int)Q, 0, 0, NTMAX))) return rc;
+  if ((rc = make_map(&m_w1, v.base + v.off[0], H / 2, H / 2, I, v.record_bytes, v.n_slots, BM, BKB))) return rc;
+  if ((rc = make_map(&m_w3, v.base + v.off[4], H / 2, H / 2, I, v.record_bytes, v.n_slots, BM, BKB))) return rc;
+  if ((rc = make_map(&m_w2, v.base + v.off[2], I / 2, I / 2, H, v.record_bytes, v.n_slots, BM, BKB))) return rc;
+  if ((rc = make_map(&m_x, s.x_codes, H / 2, H / 2, (int)Q, 0, 0, NTMAX, BKB))) return rc;
+  if ((rc = make_map(&m_h, s.h_codes, I / 2, I / 2, (int)Q, 0, 0, NTMAX, BKB))) return rc;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1033,7 +972,7 @@ int launch_decode_tc(const BankView& v, const void* x_bf16, const int32_t* slots
   const int H = v.hidden, R = rows * k;
   const DecodeScratch s = carve_decode(static_cast<uint8_t*>(workspace), H, v.inter, (size_t)R);
   const int threads = R < 1024 ? ((R + 31) / 32) * 32 : 1024;
-  decode_plan_kernel<<<1, threads, 2 * R * sizeof(int32_t), stream>>>(slots, gate_w, R, k, v.n_slots, s.seg_off, s.seg_slot, s.inv, s.src_token,
+  decode_plan_kernel<<<1, threads, 2 * R * sizeof(int32_t), stream>>>(slots, gate_w, R, k, v.n_slots, DTERMS, s.seg_off, s.seg_slot, s.inv, s.src_token,
                                                                     s.row_w, status);
   residual_quant(x_bf16, s, R, H, stream);
   int rc = run_terms4(v, s, s.seg_off, s.seg_slot, R, (long long)R * DTERMS, limit, round_bf16, status, stream);
@@ -1068,7 +1007,7 @@ int launch_prefill_exact(const BankView& v, const void* x_bf16, const int32_t* p
   if (e == cudaSuccess) e = cudaMemsetAsync(s.src_token, 0, R * 4, stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(s.row_w, 0, R * 4, stream);
   if (e != cudaSuccess) return fail(CACHALOT_ECUDA, "moe_prefill: %s", cudaGetErrorString(e));
-  plan_rows_kernel<<<n_experts, 128, 0, stream>>>(perm, offsets, slot_of_expert, v.n_slots, k, gate_w, s.inv, s.src_token, s.row_w, status);
+  plan_rows_kernel<<<n_experts, 128, 0, stream>>>(perm, offsets, slot_of_expert, v.n_slots, k, gate_w, false, s.inv, s.src_token, s.row_w, status);
   scale_offsets_kernel<<<(n_experts + 256) / 256, 256, 0, stream>>>(offsets, n_experts + 1, DTERMS, s.seg_off);
   int rc;
   if ((rc = check_launch("moe_prefill plan rows"))) return rc;
@@ -1101,12 +1040,12 @@ int launch_prefill_rows(const BankView& v, const uint8_t* x_codes, const uint8_t
   const RowScratch s = carve_rows(static_cast<uint8_t*>(workspace), I, (size_t)rows, n_seg);
   CUtensorMap m_w1, m_w3, m_w2, m_x, m_h;
   int rc;
-  if ((rc = make_map(&m_w1, v.base + v.off[0], H / 2, H / 2, I, v.record_bytes, v.n_slots, BM))) return rc;
-  if ((rc = make_map(&m_w3, v.base + v.off[4], H / 2, H / 2, I, v.record_bytes, v.n_slots, BM))) return rc;
-  if ((rc = make_map(&m_w2, v.base + v.off[2], I / 2, I / 2, H, v.record_bytes, v.n_slots, BM))) return rc;
-  if ((rc = make_map(&m_x, x_codes, H / 2, H / 2, (int)rows, 0, 0, NTMAX))) return rc;
-  if ((rc = make_map(&m_h, s.h_codes, I / 2, I / 2, (int)rows, 0, 0, NTMAX))) return rc;
-  plan_units_kernel<<<1, 256, 256 * sizeof(int32_t), stream>>>(seg_offsets, seg_slot, n_seg, v.n_slots, s.units, s.n_units);
+  if ((rc = make_map(&m_w1, v.base + v.off[0], H / 2, H / 2, I, v.record_bytes, v.n_slots, BM, BKB))) return rc;
+  if ((rc = make_map(&m_w3, v.base + v.off[4], H / 2, H / 2, I, v.record_bytes, v.n_slots, BM, BKB))) return rc;
+  if ((rc = make_map(&m_w2, v.base + v.off[2], I / 2, I / 2, H, v.record_bytes, v.n_slots, BM, BKB))) return rc;
+  if ((rc = make_map(&m_x, x_codes, H / 2, H / 2, (int)rows, 0, 0, NTMAX, BKB))) return rc;
+  if ((rc = make_map(&m_h, s.h_codes, I / 2, I / 2, (int)rows, 0, 0, NTMAX, BKB))) return rc;
+  plan_units_kernel<<<1, 256, 256 * sizeof(int32_t), stream>>>(seg_offsets, seg_slot, n_seg, v.n_slots, NTMAX, s.units, s.n_units);
   if (zero_absent) zero_absent_rows_kernel<<<n_seg, 256, 0, stream>>>(seg_offsets, seg_slot, v.n_slots, H, y);
   if ((rc = check_launch("moe_prefill plan"))) return rc;
 
@@ -1155,9 +1094,12 @@ int launch_prefill_rows(const BankView& v, const uint8_t* x_codes, const uint8_t
   return check_launch("moe_prefill down (tcgen05)");
 }
 
-int launch_combine_rows(const __nv_bfloat16* y, const int32_t* inv, int tokens, int k, int hidden, float* out, cudaStream_t stream) {
+int launch_combine_rows(const __nv_bfloat16* y, const int32_t* inv, int tokens, int k, int hidden, void* out, int out_dtype, cudaStream_t stream) {
   if (tokens <= 0) return CACHALOT_OK;
-  combine_kernel<<<tokens, 256, 0, stream>>>(y, inv, k, hidden, out);
+  if (out_dtype == CACHALOT_BF16)
+    combine_kernel<<<tokens, 256, 0, stream>>>(y, inv, k, hidden, static_cast<__nv_bfloat16*>(out));
+  else
+    combine_kernel<<<tokens, 256, 0, stream>>>(y, inv, k, hidden, static_cast<float*>(out));
   return check_launch("moe_prefill combine");
 }
 
@@ -1172,7 +1114,7 @@ int launch_prefill_tc(const BankView& v, const void* x_bf16, const int32_t* perm
   if (e == cudaSuccess) e = cudaMemsetAsync(s.src_token, 0, rows * 4, stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(s.row_w, 0, rows * 4, stream);
   if (e != cudaSuccess) return fail(CACHALOT_ECUDA, "moe_prefill: memset: %s", cudaGetErrorString(e));
-  plan_rows_kernel<<<n_experts, 128, 0, stream>>>(perm, offsets, slot_of_expert, v.n_slots, k, gate_w, s.inv, s.src_token, s.row_w,
+  plan_rows_kernel<<<n_experts, 128, 0, stream>>>(perm, offsets, slot_of_expert, v.n_slots, k, gate_w, false, s.inv, s.src_token, s.row_w,
                                                  status);
   int rc;
   if ((rc = check_launch("moe_prefill plan rows"))) return rc;
@@ -1181,7 +1123,7 @@ int launch_prefill_tc(const BankView& v, const void* x_bf16, const int32_t* perm
   if ((rc = launch_prefill_rows(v, s.x_codes, s.x_scales, s.row_w, offsets, slot_of_expert, n_experts, (long long)rows, limit, false,
                                 s.rows_ws, s.y, status, stream)))
     return rc;
-  return launch_combine_rows(s.y, s.inv, tokens, k, H, out, stream);
+  return launch_combine_rows(s.y, s.inv, tokens, k, H, out, CACHALOT_F32, stream);
 }
 
 }  // namespace cachalot

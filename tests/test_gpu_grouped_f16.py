@@ -1,0 +1,120 @@
+"""GPU parity of the grouped f16 tensor-core kernels (several tokens over a 2-bit bank) against the float64 oracle: rows that
+start in mid-group, group 64, tiles and stages that end early, units of 1, 64 and 65 rows, absent experts, more routed rows
+than one plan takes."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from oracle import affine, configs  # noqa: E402
+from tests.helpers import bf16_tensor, make_bank, within_bf16_flips  # noqa: E402
+
+
+def _bank(rng, hidden, inter, n_exp, group):
+    import cachalot_b200 as cb
+
+    experts = []
+    for _ in range(n_exp):
+        e = {}
+        for p, (n, k) in (("w1", (inter, hidden)), ("w2", (hidden, inter)), ("w3", (inter, hidden))):
+            groups = n * k // group
+            s = (rng.uniform(0.5, 1.5, groups) / np.sqrt(k)).astype(np.float16)
+            e[f"{p}.weight"] = affine.pack_bits(rng.integers(0, 4, (n, k), dtype=np.uint8), 2)
+            e[f"{p}.scales"] = s
+            e[f"{p}.biases"] = (-1.5 * s.astype(np.float32) + rng.normal(0, 0.2, groups) / np.sqrt(k)).astype(np.float16)
+        experts.append(e)
+    return experts, make_bank(experts, cb.affine_format(hidden, inter, 2, group), hidden, inter)
+
+
+def _want(x, slots, w, experts, group):
+    out = np.zeros(x.shape, np.float32)
+    for t in range(x.shape[0]):
+        for j in range(slots.shape[1]):
+            if slots[t, j] >= 0:
+                out[t] += affine.affine_expert_forward(x[t], experts[slots[t, j]], bits=2, group_size=group, weight=w[t, j], swiglu_limit=10.0,
+                                                       acc=np.float64)
+    return out
+
+
+@pytest.mark.parametrize("hidden,inter,group", [(128, 64, 64), (256, 192, 128), (512, 320, 64), (1088, 448, 128), (640, 2880, 128)])
+@pytest.mark.parametrize("tokens", [2, 17, 66])
+def test_batch(hidden, inter, group, tokens):
+    import torch
+
+    import cachalot_b200 as cb
+
+    rng = np.random.default_rng(hidden + inter + tokens)
+    experts, bank = _bank(rng, hidden, inter, 5, group)
+    x = configs.round_bf16((rng.standard_normal((tokens, hidden)) * np.exp(rng.uniform(-6, 6, (tokens, 1)))).astype(np.float32))
+    # expert 0 takes every token (66: a unit of 64 and one of 2), the others some, one route slot in seven is absent
+    slots = np.stack([np.zeros(tokens, np.int32), rng.integers(1, 5, tokens, dtype=np.int32)], 1)
+    slots[::7, 1] = -1
+    w = rng.uniform(0.1, 1.0, slots.shape).astype(np.float32)
+    want = _want(x, slots, w, experts, group)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    args = (bf16_tensor(x), torch.from_numpy(slots).cuda(), torch.from_numpy(w).cuda(), bank)
+    got = cb.moe_forward(*args, status=status)
+    assert int(status.item()) == 0
+    for t in range(tokens):  # rows differ in size: each against its own largest value
+        assert within_bf16_flips(got[t].cpu().numpy(), want[t]), f"token {t}"
+    assert torch.equal(cb.moe_forward(*args, out_dtype=torch.bfloat16), got.to(torch.bfloat16))
+
+
+def test_more_rows_than_one_plan():
+    import torch
+
+    import cachalot_b200 as cb
+
+    rng = np.random.default_rng(7)
+    experts, bank = _bank(rng, 256, 128, 3, 128)
+    x = configs.round_bf16(rng.standard_normal((1100, 256)).astype(np.float32))
+    slots = rng.integers(0, 3, (1100, 1), dtype=np.int32)
+    w = rng.uniform(0.1, 1.0, slots.shape).astype(np.float32)
+    got = cb.moe_forward(bf16_tensor(x), torch.from_numpy(slots).cuda(), torch.from_numpy(w).cuda(), bank).cpu().numpy()
+    assert within_bf16_flips(got, _want(x, slots, w, experts, 128))
+
+
+@pytest.mark.parametrize("tokens", [3, 200])
+def test_prefill(tokens):
+    import torch
+
+    import cachalot_b200 as cb
+
+    rng = np.random.default_rng(tokens)
+    experts, bank = _bank(rng, 384, 320, 8, 128)
+    bank.slot_table[0, 3] = -1
+    x = configs.round_bf16(rng.standard_normal((tokens, 384)).astype(np.float32))
+    ids = np.stack([rng.permutation(8)[:3] for _ in range(tokens)]).astype(np.int32)
+    w = rng.uniform(0.1, 1.0, ids.shape).astype(np.float32)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = cb.moe_prefill_grouped(bf16_tensor(x), torch.from_numpy(ids).cuda(), torch.from_numpy(w).cuda(), bank, status=status).cpu().numpy()
+    assert int(status.item()) == 0
+    assert within_bf16_flips(got, _want(x, np.where(ids == 3, -1, ids), w, experts, 128))
+
+
+def test_accumulation_is_exact_on_integers():
+    """Weights -1, 0, 1, 2 and small integer activations: every sum is a whole number below 2**24, so gate and up come out
+    exactly and an identity-like down projection shows them to the last bit."""
+    import torch
+
+    import cachalot_b200 as cb
+
+    rng = np.random.default_rng(3)
+    hidden, inter = 256, 128
+    e = {}
+    lev = {"w1": np.zeros((inter, hidden), np.uint8), "w3": rng.integers(0, 4, (inter, hidden), dtype=np.uint8),
+           "w2": np.where(np.eye(hidden, inter, dtype=np.uint8) > 0, 2, 1).astype(np.uint8)}
+    lev["w1"][:] = 1
+    lev["w1"][:, 0] = 3  # gate = 2 x[0] = 64 for every unit
+    for p, n in (("w1", inter * hidden), ("w2", inter * hidden), ("w3", inter * hidden)):
+        e[f"{p}.weight"] = affine.pack_bits(lev[p], 2)
+        e[f"{p}.scales"], e[f"{p}.biases"] = np.ones(n // 128, np.float16), -np.ones(n // 128, np.float16)
+    bank = make_bank([e], cb.affine_format(hidden, inter), hidden, inter)
+    x = rng.integers(-3, 4, (9, hidden)).astype(np.float32)
+    x[:, 0] = 32
+    u = configs.round_bf16(x @ (lev["w3"].astype(np.float32) - 1).T)
+    want = np.zeros((9, hidden), np.float32)
+    want[:, :inter] = configs.round_bf16(np.float32(64) * u)
+    got = cb.moe_forward(bf16_tensor(x), torch.zeros((9, 1), dtype=torch.int32, device="cuda"), torch.ones((9, 1), device="cuda"), bank,
+                         swiglu_limit=0.0).cpu().numpy()
+    assert np.array_equal(got, want)
