@@ -18,11 +18,12 @@
 // What bounds it: an expert's 2-bit rows at 6.5 TB/s leave an SM 89 cycles per 128 x 64 codes, and unpacking them
 // takes 100 instructions of each of four warps (one and + or, one FMA, one multiply per two codes); the MMAs of a
 // unit of 64 rows take 128.  So the unpacked operand goes registers -> TMEM (tcgen05.st, 32 cycles a tile), not
-// through shared memory, where writing and reading it again would take 256 cycles, and eight warps unpack.
+// through shared memory, where writing and reading it again would take 256 cycles.  A warp alone takes 330 to 470 cycles
+// for its step, most of it latency (codes from shared memory, store to TMEM): sixteen warps unpack, four per scheduler.
 //
-// Warp roles (512 threads): warp 0 TMA (weight tiles through a 3-D map {K/4 bytes, rows, slot}, activation rows
-// sixteen at a time), warp 1 owns TMEM and issues the MMAs, warps 4-11 unpack (two per TMEM lane quarter), warps
-// 12-15 drain.  Every wait is bounded (CACHALOT_STATUS_WAIT_EXPIRED).
+// Warp roles (768 threads): warp 0 TMA (weight tiles through a 3-D map {K/4 bytes, rows, slot}, activation rows
+// sixteen at a time), warp 1 owns TMEM and issues the MMAs, warps 4-19 unpack (four per TMEM lane quarter),
+// warps 20-23 drain.  Every wait is bounded (CACHALOT_STATUS_WAIT_EXPIRED).
 #include "tensor_core.cuh"
 
 namespace cachalot {
@@ -34,10 +35,11 @@ constexpr int KST = 256;          // codes of K per shared-memory stage
 constexpr int W_TILE = BM * KST / 4;
 constexpr int X_PIECE = NT * 128;  // 64 fp16 of every row
 constexpr int X_BOX = 16 * 128;    // one TMA box: 16 rows
-constexpr int NTHREADS = 512;
+constexpr int NTHREADS = 768;
+constexpr int UNPACK0 = 4, DRAIN0 = 20;  // first unpacking and draining warp
 constexpr int TMEM_COLS = 512;
 constexpr int A_COL = 256;        // operand slots start behind the accumulators
-constexpr int MAX_STAGES = 5, BAR_BYTES = 256;
+constexpr int MAX_STAGES = 5, BAR_BYTES = 512;
 constexpr int A_SLOTS = 4;        // of 64 columns: gate and up of one 64-code step, or two steps of down
 
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t tacc, uint32_t ta, uint64_t db, uint32_t idesc, uint32_t accumulate) {
@@ -130,7 +132,8 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
   uint64_t* a_empty = a_full + A_SLOTS;
   uint64_t* acc_full = a_empty + A_SLOTS;
   uint64_t* acc_empty = acc_full + 2;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* sc_full = acc_empty + 2;  // one per pair of unpacking warps
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sc_full + 8);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_holder + 1);
   uint8_t* sc_base = smem + (size_t)n_stage * STAGE_BYTES + BAR_BYTES;  // scales and biases of this and the next item
 
@@ -140,6 +143,7 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
     for (int s = 0; s < n_stage; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1);
     for (int s = 0; s < A_SLOTS; ++s) mbar_init(&a_full[s], 8), mbar_init(&a_empty[s], 1);
     for (int b = 0; b < 2; ++b) mbar_init(&acc_full[b], 1), mbar_init(&acc_empty[b], 4);
+    for (int b = 0; b < 8; ++b) mbar_init(&sc_full[b], 2);
     *abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -245,17 +249,19 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
         if (ok) tc_commit(&acc_full[buf]);
       }
     }
-  } else if (warp >= 4 && warp < 12) {
+  } else if (warp >= UNPACK0 && warp < DRAIN0) {
     // ---- codes -> fp16 operand in TMEM -----------------------------------------------------------
-    const int q = warp & 3, p = (warp - 4) >> 2;  // TMEM lane quarter; matrix (gate/up) or step parity (down)
+    // TMEM lane quarter; matrix (gate/up) or step of a slot (down); which of every two operand slots
+    const int q = warp & 3, p = ((warp - UNPACK0) >> 2) & 1, hh = (warp - UNPACK0) >> 3;
     const int m = q * 32 + lane;                  // row of the tile
-    constexpr int NS = NA == 2 ? 4 : 2;           // steps of a stage this warp unpacks
     const int sh = A.group == 128 ? 1 : 0;        // groups per 64 codes: one or a half
     const uint32_t t_dst = tmem + A_COL + ((uint32_t)(q * 32) << 16) + p * 32;
-    // A thread's scales and biases of the next item come by 16-byte asynchronous copies (a row of them starts at any even
-    // address) into windows [buffer][set][array][window][row], read back by the same thread.
+    // The scales and biases of the next item come by 16-byte asynchronous copies (a row of them starts at any even
+    // address) into windows [buffer][set][array][window][row].  The two warps that unpack the same rows (hh) share them:
+    // one brings the scales, the other the biases.
+    const long long off_s = NA == 2 && p ? A.off_s[1] : A.off_s[0], off_b = NA == 2 && p ? A.off_b[1] : A.off_b[0];
     struct RowRef {
-      const uint8_t* buf;
+      uint32_t buf;        // shared-memory address
       int lead_s, lead_b;  // halfs in front of the row's first group
       int i0;              // the row's first 64-code step, counted over the matrix
       bool ok;             // the row exists
@@ -267,19 +273,19 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
       const int n = (int)(w % n_mt) * BM + m;
       r.ok = n < A.n_rows;
       r.i0 = n * n64;
-      uint8_t* dst = sc_base + ((size_t)((par * 2 + p) * 2) * A.n_win * BM + m) * 16;
+      const uint32_t dst = smem_u32(sc_base) + (uint32_t)((par * 2 + p) * 2 * A.n_win * BM + m) * 16;
       r.buf = dst;
       const long long g0 = r.i0 >> sh, g1 = (r.i0 + n64 - 1) >> sh;
 #pragma unroll
       for (int arr = 0; arr < 2; ++arr) {
-        const uintptr_t at = reinterpret_cast<uintptr_t>(rec + (arr ? A.off_b : A.off_s)[NA == 2 ? p : 0] + 2 * g0);
+        const uintptr_t at = reinterpret_cast<uintptr_t>(rec + (arr ? off_b : off_s) + 2 * g0);
         const uintptr_t end = at + 2 * (g1 - g0 + 1);
         (arr ? r.lead_b : r.lead_s) = (int)(at & 15) >> 1;
-        if (r.ok)
+        if (r.ok && arr == hh)
           for (int i = 0; i < A.n_win; ++i) {
             const uintptr_t from = (at & ~(uintptr_t)15) + 16 * i;
             if (from < end)
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + (size_t)(arr * A.n_win + i) * BM * 16)), "l"(from) : "memory");
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)((arr * A.n_win + i) * BM * 16)), "l"(from) : "memory");
           }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
@@ -288,7 +294,9 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
     // half number i of the row's scales (arr 0) or biases (1)
     auto value = [&](const RowRef& r, int arr, int i) -> uint32_t {
       const int h = (arr ? r.lead_b : r.lead_s) + i;
-      return *reinterpret_cast<const uint16_t*>(r.buf + (size_t)(arr * A.n_win + (h >> 3)) * BM * 16 + (h & 7) * 2);
+      uint16_t v;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(r.buf + (uint32_t)((arr * A.n_win + (h >> 3)) * BM * 16 + (h & 7) * 2)));
+      return v;
     };
     const int blk_sh = (A.group == 128 && K.block == 64) ? 1 : 0;
     const int blk_per = K.block / 64;  // 64-code steps per block
@@ -300,25 +308,21 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
     };
     int s = 0, a = 0;
     uint32_t ph = 0, aph = 1;  // the first pass over the slots finds them free
-    bool ok = true, pending = false;
-    int prev = 0;
-    // Completing a store is waited for only after the next step has been unpacked
+    bool ok = true;
+    // one operand slot: free -> unpacked -> published
+    auto begin = [&]() -> bool {
+      if (!__all_sync(0xffffffffu, mbar_wait(&a_empty[a], aph, abort))) return false;
+      tc_fence_after();
+      return true;
+    };
     auto publish = [&]() {
-      if (!pending) return;
       tc_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&a_full[prev]);
-      pending = false;
+      if (lane == 0) mbar_arrive(&a_full[a]);
     };
-    auto store = [&](const uint32_t (&r)[32], bool have) -> bool {
-      publish();
-      if (!__all_sync(0xffffffffu, mbar_wait(&a_empty[a], aph, abort))) return false;
-      tc_fence_after();
-      if (have) tc_st32(t_dst + a * 64, r);
-      pending = true, prev = a;
+    auto next_slot = [&]() {
       if (++a == A_SLOTS) a = 0, aph ^= 1u;
-      return true;
     };
     RowRef cur = {}, nxt = {};
     int par = 0;
@@ -326,43 +330,41 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
     for (long long w = blockIdx.x; w < total && ok; w += gridDim.x) {
       cur = nxt;
       asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sc_full[p * 4 + q]);
+      if (!__all_sync(0xffffffffu, mbar_wait(&sc_full[p * 4 + q], par, abort))) break;  // both warps: arrived, and done with the other buffer
       par ^= 1;
       if (w + gridDim.x < total) nxt = fetch(w + gridDim.x, par);
       for (int ks = 0; ks < n_st && ok; ++ks) {
         const int steps = steps_of(ks);
         if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort))) { ok = false; break; }
-        uint32_t r[32];
-        if (ks < n_main) {
-          const uint8_t* row = smem + (size_t)s * STAGE_BYTES + (NA == 2 ? p * W_TILE : 0) + m * (KST / 4);
-#pragma unroll
-          for (int i = 0; i < NS; ++i) {
-            const int step = NA == 2 ? i : 2 * i + p;
-            if ((NA == 2 ? i : 2 * i) >= steps) break;
-            const bool have = step < steps;
-            if (have) {
-              const uint4 wv = *reinterpret_cast<const uint4*>(row + ((step ^ ((m >> 1) & 3)) << 4));
+        const uint32_t row = smem_u32(smem) + s * STAGE_BYTES + (NA == 2 ? p * W_TILE : 0) + m * (KST / 4);
+        for (int i = 0; i < steps; i += (NA == 2 ? 1 : 2), next_slot()) {
+          if ((a & 1) != hh) continue;
+          const int step = NA == 2 ? i : i + p;
+          if (!begin()) { ok = false; break; }
+          if (step < steps) {
+            uint32_t r[32];
+            if (ks < n_main) {
+              uint4 wv;
+              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                           : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
+                           : "r"(row + ((step ^ ((m >> 1) & 3)) << 4)));
               const uint32_t sv = cur.ok ? value(cur, 0, ((cur.i0 + ks * 4 + step) >> sh) - (cur.i0 >> sh)) : 0u;
-              unpack64(wv, sv | (sv << 16), r);
-            }
-            if (!store(r, have)) { ok = false; break; }
-          }
-        } else {
-          for (int i = 0; i < steps && ok; i += (NA == 2 ? 1 : 2)) {
-            const int step = NA == 2 ? i : i + p;
-            const bool have = step < steps;
-            if (have) {
+              unpack64(wv, sv * 0x10001u, r);
+            } else {
               const int e0 = ((ks - n_main) * 2 + step) * 64;
 #pragma unroll
               for (int j = 0; j < 32; ++j) r[j] = ext_val(cur, e0 + 2 * j) | (ext_val(cur, e0 + 2 * j + 1) << 16);
             }
-            if (!store(r, have)) ok = false;
+            tc_st32(t_dst + a * 64, r);
           }
+          publish();
         }
         if (++s == n_stage) s = 0, ph ^= 1u;
       }
     }
-    if (ok) publish();
-  } else if (warp >= 12) {
+  } else if (warp >= DRAIN0) {
     // ---- accumulators -> h or y -------------------------------------------------------------------
     const int q = warp & 3;
     const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
