@@ -572,6 +572,182 @@ extern "C" int cachalot_fp8_act_quant(const void* x_bf16, int rows, int k, int b
   return check_launch("fp8_act_quant");
 }
 
+// ---- many tokens: tiled GEMM -------------------------------------------------------------------------
+// The same arithmetic (e4m3 mma.sync per scale block, the block's sum times both scales added in fp32) as one launch over
+// [tokens, n]: a CTA makes 128 x 128 outputs, eight warps of 64 x 32, K in 128-byte steps through four shared-memory
+// stages (16-byte cp.async, chunks XOR-swizzled by row against ldmatrix conflicts).  What bounds it: per warp and 32
+// codes of K sixteen MMAs next to 64 FMAs that apply the scales and six ldmatrix, so issue slots before the tensor pipe.
+// The 64-token kernel above reads every weight again per 64 tokens, straight from L2 into registers: shared expert of
+// 1000 tokens, 5120 x 2304, 2729 us there, 426 us here.
+constexpr int GM_T = 128, GM_N = 128, GM_K = 128, GM_STAGES = 4, GM_THREADS = 256;
+constexpr int GM_STAGE_BYTES = (GM_T + GM_N) * GM_K + GM_T * 4 * 4 + 64;  // tiles, activation scales [4][128], weight scales [4][4]
+constexpr size_t GM_SMEM = (size_t)GM_STAGES * GM_STAGE_BYTES;
+
+__device__ __forceinline__ void gm_cp16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void gm_cp4(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void gm_ldsm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+template <int BLOCK, typename OutT>
+__global__ void __launch_bounds__(GM_THREADS, 1)
+fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act_scales, const uint8_t* __restrict__ weight,
+                const void* __restrict__ w_scales, int scale_rule, int rows, int n_out, int k, OutT* __restrict__ out, long long ldo,
+                const float* __restrict__ addend) {
+  constexpr int BPS = GM_K / BLOCK;   // scale blocks per stage: 4 or 1
+  constexpr int MPB = BLOCK / 32;     // MMAs per scale block
+  constexpr int NBW = GM_N / BLOCK;   // weight-scale rows of a tile
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int t0 = blockIdx.x * GM_T, n0 = blockIdx.y * GM_N;
+  const int wt = (warp & 1) * 64, wn = (warp >> 1) * 32;  // the warp's corner in the tile
+  const int nkb = k / BLOCK, nk = (k + GM_K - 1) / GM_K, nsr = (n_out + BLOCK - 1) / BLOCK;
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+  auto w_scale = [&](int kt) {  // weight scale number tid (row tid / BPS, block tid % BPS) of step kt
+    const int r = n0 / BLOCK + tid / BPS, kb = kt * BPS + tid % BPS;
+    if (r >= nsr || kb >= nkb) return 0.f;
+    const size_t i = (size_t)r * nkb + kb;
+    return scale_rule == CACHALOT_SCALE_E8M0 ? e8m0_to_f32(__ldg(reinterpret_cast<const uint8_t*>(w_scales) + i))
+                                             : __ldg(reinterpret_cast<const float*>(w_scales) + i);
+  };
+  auto load = [&](int kt) {
+    const uint32_t st = sbase + (kt % GM_STAGES) * GM_STAGE_BYTES;
+#pragma unroll
+    for (int i = 0; i < (GM_T + GM_N) * 8 / GM_THREADS; ++i) {
+      const int id = tid + i * GM_THREADS, r = (id >> 3) & 127, c = id & 7;
+      const int kx = kt * GM_K + c * 16;
+      // rows behind the end repeat the last one and are never stored; behind the end of K zeros
+      const uint8_t* src = id < GM_T * 8 ? codes + (size_t)min(t0 + r, rows - 1) * k : weight + (size_t)min(n0 + r, n_out - 1) * k;
+      gm_cp16(st + (id < GM_T * 8 ? 0 : GM_T * GM_K) + r * GM_K + ((c ^ (r & 7)) << 4), src + (kx < k ? kx : 0), kx < k ? 16 : 0);
+    }
+#pragma unroll
+    for (int i = 0; i < (GM_T * BPS + GM_THREADS - 1) / GM_THREADS; ++i) {
+      const int id = tid + i * GM_THREADS, r = id & (GM_T - 1), b = id / GM_T, kb = kt * BPS + b;
+      if (id < GM_T * BPS)
+        gm_cp4(st + (GM_T + GM_N) * GM_K + id * 4, act_scales + (size_t)min(t0 + r, rows - 1) * nkb + min(kb, nkb - 1), kb < nkb ? 4 : 0);
+    }
+  };
+  const int lr = lane & 7, lm = lane >> 3;  // ldmatrix: this lane's row of matrix lm
+  float acc[4][4][4];
+  // The two NaN codes of E4M3 read as zero.  A tile runs unmasked first: a NaN weight shows as a NaN in the sums, and
+  // only then the tile is made again with the codes masked.
+  for (int masked = 0; masked < 2; ++masked) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.f;
+    float ws_next = 0.f;
+    auto put_scale = [&](int kt, float v) {
+      if (tid < NBW * BPS) *reinterpret_cast<float*>(smem + (kt % GM_STAGES) * GM_STAGE_BYTES + (GM_T + GM_N) * GM_K + GM_T * 16 + tid * 4) = v;
+    };
+#pragma unroll
+    for (int i = 0; i < GM_STAGES - 1; ++i) {
+      if (i < nk) {
+        load(i);
+        if (tid < NBW * BPS) put_scale(i, w_scale(i));
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int kt = 0; kt < nk; ++kt) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(GM_STAGES - 2) : "memory");
+      // the weight scale asked for one step ago belongs to step kt + GM_STAGES - 2: read by others only after this barrier
+      if (kt > 0 && kt + GM_STAGES - 2 < nk) put_scale(kt + GM_STAGES - 2, ws_next);
+      __syncthreads();
+      if (kt + GM_STAGES - 1 < nk) {
+        load(kt + GM_STAGES - 1);
+        if (tid < NBW * BPS) ws_next = w_scale(kt + GM_STAGES - 1);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const uint8_t* stp = smem + (kt % GM_STAGES) * GM_STAGE_BYTES;
+      const uint32_t st = sbase + (kt % GM_STAGES) * GM_STAGE_BYTES;
+      const float* s_as = reinterpret_cast<const float*>(stp + (GM_T + GM_N) * GM_K);
+      const float* s_ws = s_as + GM_T * 4;
+#pragma unroll
+      for (int b = 0; b < BPS; ++b) {
+        float d[4][4][4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) d[a][c][0] = d[a][c][1] = d[a][c][2] = d[a][c][3] = 0.f;
+#pragma unroll
+        for (int m = 0; m < MPB; ++m) {
+          const int ch = (b * MPB + m) * 2;  // first 16-byte chunk of these 32 codes
+          uint32_t wb[2][4];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {  // weight rows wn + 16c ..: {rows 0-7, 8-15} x {chunk, chunk + 1}
+            const int r = wn + c * 16 + (lm >> 1) * 8 + lr;
+            gm_ldsm4(wb[c], st + GM_T * GM_K + r * GM_K + (((ch + (lm & 1)) ^ (r & 7)) << 4));
+            if (masked) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) wb[c][i] = e4m3x4_nan_to_zero(wb[c][i]);
+            }
+          }
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            uint32_t xa[4];
+            const int r = wt + a * 16 + (lm & 1) * 8 + lr;
+            gm_ldsm4(xa, st + r * GM_K + (((ch + (lm >> 1)) ^ (r & 7)) << 4));
+#pragma unroll
+            for (int c = 0; c < 4; ++c) qmma_e4m3(d[a][c], xa[0], xa[1], xa[2], xa[3], wb[c >> 1][(c & 1) * 2], wb[c >> 1][(c & 1) * 2 + 1]);
+          }
+        }
+        const float ws = s_ws[(BLOCK == 32 ? wn / 32 : 0) * BPS + b];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const float s0 = s_as[b * GM_T + wt + a * 16 + g] * ws, s1 = s_as[b * GM_T + wt + a * 16 + g + 8] * ws;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            acc[a][c][0] = fmaf(d[a][c][0], s0, acc[a][c][0]);
+            acc[a][c][1] = fmaf(d[a][c][1], s0, acc[a][c][1]);
+            acc[a][c][2] = fmaf(d[a][c][2], s1, acc[a][c][2]);
+            acc[a][c][3] = fmaf(d[a][c][3], s1, acc[a][c][3]);
+          }
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float chk = 0.f;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) chk += (acc[a][c][0] + acc[a][c][1]) + (acc[a][c][2] + acc[a][c][3]);
+    if (!__syncthreads_or(chk != chk)) break;
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int tok = t0 + wt + a * 16 + g + (i >> 1) * 8;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int row = n0 + wn + c * 8 + 2 * t + (i & 1);
+        if (tok >= rows || row >= n_out) continue;
+        float v = acc[a][c][i];
+        if (addend) v = bf16_round(v) + addend[(size_t)tok * n_out + row];
+        if constexpr (sizeof(OutT) == 2)
+          out[(size_t)tok * ldo + row] = __float2bfloat16_rn(v);
+        else
+          out[(size_t)tok * ldo + row] = v;
+      }
+    }
+}
+
+template <typename OutT>
+static cudaError_t launch_gemm(int block, cudaStream_t s, const uint8_t* codes, const float* act_scales, const uint8_t* weight,
+                               const void* w_scales, int scale_rule, int rows, int n, int k, OutT* out, long long ldo, const float* addend) {
+  const dim3 grid((rows + GM_T - 1) / GM_T, (n + GM_N - 1) / GM_N);
+  auto go = [&](auto kern) {
+    const cudaError_t e = smem_optin_once(kern, (int)GM_SMEM);
+    if (e == cudaSuccess) kern<<<grid, GM_THREADS, GM_SMEM, s>>>(codes, act_scales, weight, w_scales, scale_rule, rows, n, k, out, ldo, addend);
+    return e;
+  };
+  return block == 32 ? go(fp8_gemm_kernel<32, OutT>) : go(fp8_gemm_kernel<128, OutT>);
+}
+
 // pdl: the kernel directly before this call in the stream is one of this file's quantisers (it writes the codes and
 // scales only), so the GEMV may start streaming weights while it runs
 static int gemv_checked(const char* who, const uint8_t* codes, const float* act_scales, const uint8_t* weight, const void* w_scales,
@@ -585,7 +761,15 @@ static int gemv_checked(const char* who, const uint8_t* codes, const float* act_
   if (!aligned(weight, 8) || !aligned(codes, 8) || k % 8) return fail(CACHALOT_EALIGN, "%s: weight and codes need 8-byte alignment", who);
   if (ldo < n) return fail(CACHALOT_EINVAL, "%s: output row pitch %lld < %d", who, ldo, n);
   if (rows == 0) return CACHALOT_OK;
-  // 64 tokens per launch; more tokens take more launches over the same weights
+  // More tokens than one launch of the kernels below takes: the tiled GEMM (its 16-byte copies need 16-byte rows)
+  if (rows > 8 * GEMV_MAX_TG && aligned(weight, 16) && aligned(codes, 16) && k % 16 == 0 && (n + GM_N - 1) / GM_N <= 65535) {
+    const cudaError_t e = out_dtype == CACHALOT_BF16
+                              ? launch_gemm(block, s, codes, act_scales, weight, w_scales, scale_rule, rows, n, k, (__nv_bfloat16*)out, ldo, addend)
+                              : launch_gemm(block, s, codes, act_scales, weight, w_scales, scale_rule, rows, n, k, (float*)out, ldo, addend);
+    if (e != cudaSuccess) return fail(CACHALOT_ECUDA, "%s: %s", who, cudaGetErrorString(e));
+    return check_launch(who);
+  }
+  // 64 tokens per launch; more tokens (of rows that are not 16-byte aligned) take more launches over the same weights
   for (int r0 = 0; r0 < rows; r0 += 8 * GEMV_MAX_TG) {
     const int nr = rows - r0 < 8 * GEMV_MAX_TG ? rows - r0 : 8 * GEMV_MAX_TG;
     const int ntg = (nr + 7) / 8;
