@@ -471,9 +471,8 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 }  // namespace cachalot
 
-extern "C" size_t cachalot_moe_prefill_workspace_bytes(const cachalot_bank_desc* desc, int tokens, int k,
-                                                       int mxfp4_act) {
-  if (!desc || tokens <= 0 || k <= 0) return 0;
+// what moe_prefill cannot do without; with less than cachalot_moe_prefill_workspace_bytes a 2-bit bank goes token by token
+static size_t prefill_min_workspace(const cachalot_bank_desc* desc, int tokens, int k, int mxfp4_act) {
   size_t rows = (size_t)tokens * k;
   // the tensor-core path (what prefill_tc_supported() accepts, stated on the descriptor) needs its own scratch only
   const bool tc_shape = desc->format == CACHALOT_BANK_FP4 && desc->hidden % 128 == 0 && desc->inter % 64 == 0 && desc->record_bytes % 16 == 0;
@@ -484,17 +483,21 @@ extern "C" size_t cachalot_moe_prefill_workspace_bytes(const cachalot_bank_desc*
   size_t b = align_up(rows * desc->inter * sizeof(float), 256);   // hidden
   b += align_up(rows * sizeof(int32_t), 256);                     // slot per routed row
   if (mxfp4_act) b += align_up((size_t)tokens * desc->hidden * 2, 256);  // MXFP4-rounded x as bf16
-  const BankView v = shape_view(desc);
-  if (!mxfp4_act && f16_supported(v) && rows <= 65535) {  // the expert count is not known here
-    const size_t f = prefill_f16_workspace_bytes(v, tokens, k, 8192);
-    if (f > b) b = f;
-  }
   if (mxfp4_act == 1 && desc->format == CACHALOT_BANK_FP4) {
     // experts without rows get no unit, so the unit list is bounded by the rows whatever the number of experts is
     const size_t tc = prefill_tc_workspace_bytes(desc->hidden, desc->inter, tokens, k, tokens * k);
     if (tc > b) b = tc;
   }
   return b;
+}
+
+extern "C" size_t cachalot_moe_prefill_workspace_bytes(const cachalot_bank_desc* desc, int tokens, int k, int mxfp4_act) {
+  if (!desc || tokens <= 0 || k <= 0) return 0;
+  const size_t b = prefill_min_workspace(desc, tokens, k, mxfp4_act);
+  const BankView v = shape_view(desc);
+  if (mxfp4_act || !f16_supported(v) || (long long)tokens * k > 65535) return b;
+  const size_t f = prefill_f16_workspace_bytes(v, tokens, k, 8192);  // the expert count is not known here
+  return f > b ? f : b;
 }
 
 extern "C" int cachalot_moe_prefill(const void* bank, const cachalot_bank_desc* desc, const void* x_bf16,
@@ -513,7 +516,7 @@ extern "C" int cachalot_moe_prefill(const void* bank, const cachalot_bank_desc* 
   if ((long long)tokens * k > 0x7fffffffLL) return fail(CACHALOT_EINVAL, "moe_prefill: tokens*k=%lld is too large", (long long)tokens * k);
   // the per-row kernels index routed rows in a grid dimension; the tensor-core path has no such limit
   if (!tc && (long long)tokens * k > 65535) return fail(CACHALOT_EINVAL, "moe_prefill: tokens*k=%lld exceeds 65535 (chunk the prompt)", (long long)tokens * k);
-  size_t need = cachalot_moe_prefill_workspace_bytes(desc, tokens, k, mxfp4_act);
+  const size_t need = prefill_min_workspace(desc, tokens, k, mxfp4_act);
   if (!workspace || workspace_bytes < need) return fail(CACHALOT_ESCRATCH, "moe_prefill: workspace %zu < %zu bytes", workspace_bytes, need);
   if (!aligned(workspace, 256)) return fail(CACHALOT_EALIGN, "moe_prefill: workspace must be 256-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
@@ -523,7 +526,8 @@ extern "C" int cachalot_moe_prefill(const void* bank, const cachalot_bank_desc* 
   if (tc)
     return launch_prefill_tc(v, x_bf16, perm, offsets, slot_of_expert, gate_w, tokens, k, n_experts, swiglu_limit, workspace, out,
                              status, s);
-  if (!mxfp4_act && f16_supported(v) && n_experts <= 8192 && grouped_f16_pays(rows, n_experts))
+  if (!mxfp4_act && f16_supported(v) && n_experts <= 8192 && grouped_f16_pays(rows, n_experts) &&
+      workspace_bytes >= prefill_f16_workspace_bytes(v, tokens, k, n_experts))
     return launch_prefill_f16(v, x_bf16, perm, offsets, slot_of_expert, gate_w, tokens, k, n_experts, swiglu_limit, workspace, out, status, s);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   float* hidden = reinterpret_cast<float*>(ws);
