@@ -579,9 +579,21 @@ extern "C" int cachalot_fp8_act_quant(const void* x_bf16, int rows, int k, int b
 // codes of K sixteen MMAs next to 64 FMAs that apply the scales and six ldmatrix, so issue slots before the tensor pipe.
 // The 64-token kernel above reads every weight again per 64 tokens, straight from L2 into registers: shared expert of
 // 1000 tokens, 5120 x 2304, 2729 us there, 426 us here.
-constexpr int GM_T = 128, GM_N = 128, GM_K = 128, GM_STAGES = 4, GM_THREADS = 256;
-constexpr int GM_STAGE_BYTES = (GM_T + GM_N) * GM_K + GM_T * 4 * 4 + 64;  // tiles, activation scales [4][128], weight scales [4][4]
-constexpr size_t GM_SMEM = (size_t)GM_STAGES * GM_STAGE_BYTES;
+// Nine to 64 tokens are bound by the weights' way in: small tiles (32 tokens x 64 outputs, or 64 x 32; warps of 16 x 16)
+// that spread a 4096-row matrix over the SMs, two CTAs each, with six stages in flight:
+// 32 tokens through [12288,4096] + [4096,8192] take 81.9 us on the per-lane kernel, 75.8 here.
+constexpr int GM_K = 128, GM_THREADS = 256;
+template <int T, int N, int WT, int WN, int STAGES>
+struct GmTile {
+  static constexpr int t = T, n = N, wt = WT, wn = WN, stages = STAGES;
+  static constexpr int warps_t = T / WT;
+  static constexpr int stage_bytes = (T + N) * GM_K + T * 16;  // tiles, activation scales [4][T]
+  static constexpr size_t smem = (size_t)STAGES * stage_bytes;
+  static_assert((T / WT) * (N / WN) * 32 == GM_THREADS, "eight warps");
+};
+using GmLarge = GmTile<128, 128, 64, 32, 4>;
+using GmMid = GmTile<64, 32, 16, 16, 6>;
+using GmSmall = GmTile<32, 64, 16, 16, 6>;
 
 __device__ __forceinline__ void gm_cp16(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -593,36 +605,41 @@ __device__ __forceinline__ void gm_ldsm4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
-template <int BLOCK, typename OutT>
-__global__ void __launch_bounds__(GM_THREADS, 1)
+template <int BLOCK, typename OutT, typename TL>
+__global__ void __launch_bounds__(GM_THREADS, TL::smem <= 110 * 1024 ? 2 : 1)
 fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act_scales, const uint8_t* __restrict__ weight,
                 const void* __restrict__ w_scales, int scale_rule, int rows, int n_out, int k, OutT* __restrict__ out, long long ldo,
                 const float* __restrict__ addend) {
+  constexpr int GM_T = TL::t, GM_N = TL::n, GM_STAGES = TL::stages, GM_STAGE_BYTES = TL::stage_bytes;
+  constexpr int MA = TL::wt / 16, NC = TL::wn / 8;  // MMA tiles of a warp
   constexpr int BPS = GM_K / BLOCK;   // scale blocks per stage: 4 or 1
   constexpr int MPB = BLOCK / 32;     // MMAs per scale block
-  constexpr int NBW = GM_N / BLOCK;   // weight-scale rows of a tile
+  constexpr int NBW = GM_N > BLOCK ? GM_N / BLOCK : 1;  // weight-scale rows of a tile (a tile of fewer rows lies in one)
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int t0 = blockIdx.x * GM_T, n0 = blockIdx.y * GM_N;
-  const int wt = (warp & 1) * 64, wn = (warp >> 1) * 32;  // the warp's corner in the tile
+  const int wt = (warp % TL::warps_t) * TL::wt, wn = (warp / TL::warps_t) * TL::wn;  // the warp's corner in the tile
   const int nkb = k / BLOCK, nk = (k + GM_K - 1) / GM_K, nsr = (n_out + BLOCK - 1) / BLOCK;
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-  auto w_scale = [&](int kt) {  // weight scale number tid (row tid / BPS, block tid % BPS) of step kt
-    const int r = n0 / BLOCK + tid / BPS, kb = kt * BPS + tid % BPS;
-    if (r >= nsr || kb >= nkb) return 0.f;
-    const size_t i = (size_t)r * nkb + kb;
-    return scale_rule == CACHALOT_SCALE_E8M0 ? e8m0_to_f32(__ldg(reinterpret_cast<const uint8_t*>(w_scales) + i))
-                                             : __ldg(reinterpret_cast<const float*>(w_scales) + i);
-  };
+  // the tile's weight scales [NBW][nkb] as fp32, brought in once: asked for step by step, each step waited for one
+  float* s_w = reinterpret_cast<float*>(smem + (size_t)GM_STAGES * GM_STAGE_BYTES);
+  for (int i = tid; i < NBW * nkb; i += GM_THREADS) {
+    const int r = n0 / BLOCK + i / nkb;
+    const size_t at = (size_t)min(r, nsr - 1) * nkb + i % nkb;
+    s_w[i] = scale_rule == CACHALOT_SCALE_E8M0 ? e8m0_to_f32(__ldg(reinterpret_cast<const uint8_t*>(w_scales) + at))
+                                               : __ldg(reinterpret_cast<const float*>(w_scales) + at);
+  }
   auto load = [&](int kt) {
     const uint32_t st = sbase + (kt % GM_STAGES) * GM_STAGE_BYTES;
 #pragma unroll
     for (int i = 0; i < (GM_T + GM_N) * 8 / GM_THREADS; ++i) {
-      const int id = tid + i * GM_THREADS, r = (id >> 3) & 127, c = id & 7;
+      const int id = tid + i * GM_THREADS, c = id & 7;
+      const bool is_x = id < GM_T * 8;
+      const int r = is_x ? id >> 3 : (id >> 3) - GM_T;
       const int kx = kt * GM_K + c * 16;
       // rows behind the end repeat the last one and are never stored; behind the end of K zeros
-      const uint8_t* src = id < GM_T * 8 ? codes + (size_t)min(t0 + r, rows - 1) * k : weight + (size_t)min(n0 + r, n_out - 1) * k;
-      gm_cp16(st + (id < GM_T * 8 ? 0 : GM_T * GM_K) + r * GM_K + ((c ^ (r & 7)) << 4), src + (kx < k ? kx : 0), kx < k ? 16 : 0);
+      const uint8_t* src = is_x ? codes + (size_t)min(t0 + r, rows - 1) * k : weight + (size_t)min(n0 + r, n_out - 1) * k;
+      gm_cp16(st + (is_x ? 0 : GM_T * GM_K) + r * GM_K + ((c ^ (r & 7)) << 4), src + (kx < k ? kx : 0), kx < k ? 16 : 0);
     }
 #pragma unroll
     for (int i = 0; i < (GM_T * BPS + GM_THREADS - 1) / GM_THREADS; ++i) {
@@ -632,53 +649,40 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
     }
   };
   const int lr = lane & 7, lm = lane >> 3;  // ldmatrix: this lane's row of matrix lm
-  float acc[4][4][4];
+  float acc[MA][NC][4];
   // The two NaN codes of E4M3 read as zero.  A tile runs unmasked first: a NaN weight shows as a NaN in the sums, and
   // only then the tile is made again with the codes masked.
   for (int masked = 0; masked < 2; ++masked) {
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < MA; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.f;
-    float ws_next = 0.f;
-    auto put_scale = [&](int kt, float v) {
-      if (tid < NBW * BPS) *reinterpret_cast<float*>(smem + (kt % GM_STAGES) * GM_STAGE_BYTES + (GM_T + GM_N) * GM_K + GM_T * 16 + tid * 4) = v;
-    };
+      for (int b = 0; b < NC; ++b) acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.f;
 #pragma unroll
     for (int i = 0; i < GM_STAGES - 1; ++i) {
-      if (i < nk) {
-        load(i);
-        if (tid < NBW * BPS) put_scale(i, w_scale(i));
-      }
+      if (i < nk) load(i);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
     for (int kt = 0; kt < nk; ++kt) {
       asm volatile("cp.async.wait_group %0;" ::"n"(GM_STAGES - 2) : "memory");
-      // the weight scale asked for one step ago belongs to step kt + GM_STAGES - 2: read by others only after this barrier
-      if (kt > 0 && kt + GM_STAGES - 2 < nk) put_scale(kt + GM_STAGES - 2, ws_next);
       __syncthreads();
-      if (kt + GM_STAGES - 1 < nk) {
-        load(kt + GM_STAGES - 1);
-        if (tid < NBW * BPS) ws_next = w_scale(kt + GM_STAGES - 1);
-      }
+      if (kt + GM_STAGES - 1 < nk) load(kt + GM_STAGES - 1);
       asm volatile("cp.async.commit_group;" ::: "memory");
       const uint8_t* stp = smem + (kt % GM_STAGES) * GM_STAGE_BYTES;
       const uint32_t st = sbase + (kt % GM_STAGES) * GM_STAGE_BYTES;
       const float* s_as = reinterpret_cast<const float*>(stp + (GM_T + GM_N) * GM_K);
-      const float* s_ws = s_as + GM_T * 4;
 #pragma unroll
       for (int b = 0; b < BPS; ++b) {
-        float d[4][4][4];
+        float d[MA][NC][4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < MA; ++a)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) d[a][c][0] = d[a][c][1] = d[a][c][2] = d[a][c][3] = 0.f;
+          for (int c = 0; c < NC; ++c) d[a][c][0] = d[a][c][1] = d[a][c][2] = d[a][c][3] = 0.f;
 #pragma unroll
         for (int m = 0; m < MPB; ++m) {
           const int ch = (b * MPB + m) * 2;  // first 16-byte chunk of these 32 codes
-          uint32_t wb[2][4];
+          uint32_t wb[NC / 2][4];
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {  // weight rows wn + 16c ..: {rows 0-7, 8-15} x {chunk, chunk + 1}
+          for (int c = 0; c < NC / 2; ++c) {  // weight rows wn + 16c ..: {rows 0-7, 8-15} x {chunk, chunk + 1}
             const int r = wn + c * 16 + (lm >> 1) * 8 + lr;
             gm_ldsm4(wb[c], st + GM_T * GM_K + r * GM_K + (((ch + (lm & 1)) ^ (r & 7)) << 4));
             if (masked) {
@@ -687,20 +691,21 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
             }
           }
 #pragma unroll
-          for (int a = 0; a < 4; ++a) {
+          for (int a = 0; a < MA; ++a) {
             uint32_t xa[4];
             const int r = wt + a * 16 + (lm & 1) * 8 + lr;
             gm_ldsm4(xa, st + r * GM_K + (((ch + (lm >> 1)) ^ (r & 7)) << 4));
 #pragma unroll
-            for (int c = 0; c < 4; ++c) qmma_e4m3(d[a][c], xa[0], xa[1], xa[2], xa[3], wb[c >> 1][(c & 1) * 2], wb[c >> 1][(c & 1) * 2 + 1]);
+            for (int c = 0; c < NC; ++c) qmma_e4m3(d[a][c], xa[0], xa[1], xa[2], xa[3], wb[c >> 1][(c & 1) * 2], wb[c >> 1][(c & 1) * 2 + 1]);
           }
         }
-        const float ws = s_ws[(BLOCK == 32 ? wn / 32 : 0) * BPS + b];
+        if (kt * BPS + b >= nkb) break;  // behind the end of K
+        const float ws = s_w[(BLOCK == 32 ? wn / 32 : 0) * nkb + kt * BPS + b];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
+        for (int a = 0; a < MA; ++a) {
           const float s0 = s_as[b * GM_T + wt + a * 16 + g] * ws, s1 = s_as[b * GM_T + wt + a * 16 + g + 8] * ws;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < NC; ++c) {
             acc[a][c][0] = fmaf(d[a][c][0], s0, acc[a][c][0]);
             acc[a][c][1] = fmaf(d[a][c][1], s0, acc[a][c][1]);
             acc[a][c][2] = fmaf(d[a][c][2], s1, acc[a][c][2]);
@@ -712,18 +717,18 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     float chk = 0.f;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < MA; ++a)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) chk += (acc[a][c][0] + acc[a][c][1]) + (acc[a][c][2] + acc[a][c][3]);
+      for (int c = 0; c < NC; ++c) chk += (acc[a][c][0] + acc[a][c][1]) + (acc[a][c][2] + acc[a][c][3]);
     if (!__syncthreads_or(chk != chk)) break;
   }
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < MA; ++a)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int tok = t0 + wt + a * 16 + g + (i >> 1) * 8;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < NC; ++c) {
         const int row = n0 + wn + c * 8 + 2 * t + (i & 1);
         if (tok >= rows || row >= n_out) continue;
         float v = acc[a][c][i];
@@ -739,13 +744,19 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
 template <typename OutT>
 static cudaError_t launch_gemm(int block, cudaStream_t s, const uint8_t* codes, const float* act_scales, const uint8_t* weight,
                                const void* w_scales, int scale_rule, int rows, int n, int k, OutT* out, long long ldo, const float* addend) {
-  const dim3 grid((rows + GM_T - 1) / GM_T, (n + GM_N - 1) / GM_N);
-  auto go = [&](auto kern) {
-    const cudaError_t e = smem_optin_once(kern, (int)GM_SMEM);
-    if (e == cudaSuccess) kern<<<grid, GM_THREADS, GM_SMEM, s>>>(codes, act_scales, weight, w_scales, scale_rule, rows, n, k, out, ldo, addend);
+  auto go = [&](auto kern, auto tile) {
+    using TL = decltype(tile);
+    const dim3 grid((rows + TL::t - 1) / TL::t, (n + TL::n - 1) / TL::n);
+    const size_t smem = TL::smem + (size_t)((TL::n + block - 1) / block) * (k / block) * 4;
+    const cudaError_t e = smem_optin_once(kern, 227 * 1024);
+    if (e == cudaSuccess) kern<<<grid, GM_THREADS, smem, s>>>(codes, act_scales, weight, w_scales, scale_rule, rows, n, k, out, ldo, addend);
     return e;
   };
-  return block == 32 ? go(fp8_gemm_kernel<32, OutT>) : go(fp8_gemm_kernel<128, OutT>);
+  auto pick = [&](auto tile) {
+    using TL = decltype(tile);
+    return block == 32 ? go(fp8_gemm_kernel<32, OutT, TL>, tile) : go(fp8_gemm_kernel<128, OutT, TL>, tile);
+  };
+  return rows <= 32 ? pick(GmSmall()) : rows <= 64 ? pick(GmMid()) : pick(GmLarge());
 }
 
 // pdl: the kernel directly before this call in the stream is one of this file's quantisers (it writes the codes and
@@ -761,8 +772,8 @@ static int gemv_checked(const char* who, const uint8_t* codes, const float* act_
   if (!aligned(weight, 8) || !aligned(codes, 8) || k % 8) return fail(CACHALOT_EALIGN, "%s: weight and codes need 8-byte alignment", who);
   if (ldo < n) return fail(CACHALOT_EINVAL, "%s: output row pitch %lld < %d", who, ldo, n);
   if (rows == 0) return CACHALOT_OK;
-  // More tokens than one launch of the kernels below takes: the tiled GEMM (its 16-byte copies need 16-byte rows)
-  if (rows > 8 * GEMV_MAX_TG && aligned(weight, 16) && aligned(codes, 16) && k % 16 == 0 && (n + GM_N - 1) / GM_N <= 65535) {
+  // More than eight tokens: the tiled GEMM (its 16-byte copies need 16-byte rows; K is bounded by the room for scales)
+  if (rows > 8 && aligned(weight, 16) && aligned(codes, 16) && k % 16 == 0 && n <= 32 * 65535 && k <= 1 << 16) {
     const cudaError_t e = out_dtype == CACHALOT_BF16
                               ? launch_gemm(block, s, codes, act_scales, weight, w_scales, scale_rule, rows, n, k, (__nv_bfloat16*)out, ldo, addend)
                               : launch_gemm(block, s, codes, act_scales, weight, w_scales, scale_rule, rows, n, k, (float*)out, ldo, addend);
@@ -780,7 +791,7 @@ static int gemv_checked(const char* who, const uint8_t* codes, const float* act_
     GsGeo G;
     bool staged = false;
     // up to eight tokens; beyond that the activation fragments outweigh the weights and the per-lane kernel, which
-    // shares them between two row tiles, is the faster one (measured at 32 tokens)
+    // shares them between two row tiles, is the faster one of the two (rows that the GEMM does not take)
     if (!no_stream && ntg == 1 && gs_geometry(nr, k, block, 1, &staged, &G)) {
       cudaError_t e;
       if (out_dtype == CACHALOT_BF16) {

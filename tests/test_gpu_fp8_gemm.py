@@ -1,4 +1,4 @@
-"""The tiled FP8 GEMM (more than 64 tokens) against the streaming GEMV (one token at a time, itself checked against the oracle):
+"""The tiled FP8 GEMM (more than eight tokens) against the streaming GEMV (one token at a time, itself checked against the oracle):
 the same products summed in fp32 in another order, at sizes that end inside a tile, a K step and a scale block row; weights
 that hold the two NaN codes, which read as zero."""
 import pytest
@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,k,rule", [(16, 32, "e8m0"), (200, 96, "e8m0"), (129, 416, "e8m0"), (384, 1184, "e8m0"), (130, 128, "f32"), (300, 640, "f32")])
-@pytest.mark.parametrize("rows", [65, 128, 300])
+@pytest.mark.parametrize("rows", [9, 32, 33, 64, 65, 300])
 @pytest.mark.parametrize("nan", [False, True])
 def test_rows_match_single_tokens(n, k, rule, rows, nan):
     import torch
