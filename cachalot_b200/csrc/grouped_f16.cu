@@ -37,6 +37,7 @@ constexpr int X_PIECE = NT * 128;  // 64 fp16 of every row
 constexpr int X_BOX = 16 * 128;    // one TMA box: 16 rows
 constexpr int NTHREADS = 768;
 constexpr int UNPACK0 = 4, DRAIN0 = 20;  // first unpacking and draining warp
+constexpr int N_UNPACK = DRAIN0 - UNPACK0;
 constexpr int TMEM_COLS = 512;
 constexpr int A_COL = 256;        // operand slots start behind the accumulators
 constexpr int MAX_STAGES = 5, BAR_BYTES = 512;
@@ -139,8 +140,10 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    // a stage is free when its last MMA is done: the unpacking warps have read it before that MMA is issued
-    for (int s = 0; s < n_stage; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1);
+    // A stage is free when its last MMA is done and every unpacking warp has passed it.  The MMAs alone do not say that:
+    // a stage with one operand slot waits for the eight warps of one set only, and a warp of the other set that came to
+    // full[s] after the next fill would take that phase for the one before its own and wait for good.
+    for (int s = 0; s < n_stage; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1 + N_UNPACK);
     for (int s = 0; s < A_SLOTS; ++s) mbar_init(&a_full[s], 8), mbar_init(&a_empty[s], 1);
     for (int b = 0; b < 2; ++b) mbar_init(&acc_full[b], 1), mbar_init(&acc_empty[b], 4);
     for (int b = 0; b < 8; ++b) mbar_init(&sc_full[b], 2);
@@ -361,6 +364,9 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
           }
           publish();
         }
+        if (!ok) break;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
         if (++s == n_stage) s = 0, ph ^= 1u;
       }
     }

@@ -60,6 +60,30 @@ def test_batch(hidden, inter, group, tokens):
     assert torch.equal(cb.moe_forward(*args, out_dtype=torch.bfloat16), got.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("hidden,inter,group", [(3136, 2880, 64), (3136, 2880, 128), (576, 320, 64)])
+def test_stages_with_one_operand_slot(hidden, inter, group):
+    """K of 4i+1 steps of 64 codes, two to four shared-memory stages, several units per CTA: stages that only half of the
+    unpacking warps work on are filled again only when the other half has passed them too."""
+    import torch
+
+    import cachalot_b200 as cb
+
+    rng = np.random.default_rng(hidden + group)
+    experts, bank = _bank(rng, hidden, inter, 3, group)
+    tokens = 500
+    x = configs.round_bf16(rng.standard_normal((tokens, hidden)).astype(np.float32))
+    slots = np.stack([rng.permutation(3)[:2] for _ in range(tokens)]).astype(np.int32)
+    w = rng.uniform(0.1, 1.0, slots.shape).astype(np.float32)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    args = (bf16_tensor(x), torch.from_numpy(slots).cuda(), torch.from_numpy(w).cuda(), bank)
+    got = cb.moe_forward(*args, status=status)
+    for _ in range(20):
+        assert torch.equal(cb.moe_forward(*args, status=status), got)
+    assert int(status.item()) == 0
+    some = [0, 255, tokens - 1]
+    assert within_bf16_flips(got[some].cpu().numpy(), _want(x[some], slots[some], w[some], experts, group))
+
+
 def test_more_rows_than_one_plan():
     import torch
 
