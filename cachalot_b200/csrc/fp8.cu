@@ -1,6 +1,7 @@
 // FP8 E4M3 trunk GEMV with dynamic activation quantisation (act_quant).
 #include <cuda_fp8.h>
 
+#include <cfloat>
 #include <cstdlib>
 #include <mutex>
 #include <set>
@@ -582,13 +583,17 @@ extern "C" int cachalot_fp8_act_quant(const void* x_bf16, int rows, int k, int b
 // Nine to 64 tokens are bound by the weights' way in: small tiles (32 tokens x 64 outputs, or 64 x 32; warps of 16 x 16)
 // that spread a 4096-row matrix over the SMs, two CTAs each, with six stages in flight:
 // 32 tokens through [12288,4096] + [4096,8192] take 81.9 us on the per-lane kernel, 75.8 here.
-constexpr int GM_K = 128, GM_THREADS = 256;
+constexpr int GM_K = 128, GM_THREADS = 256, GM_SMEM_LIMIT = 227 * 1024;
+// a tile's weight scales as fp32: [scale rows of the tile][K / block]
+static size_t gm_scale_bytes(int n, int k, int block) { return (size_t)((n + block - 1) / block) * (k / block) * 4; }
 template <int T, int N, int WT, int WN, int STAGES>
 struct GmTile {
   static constexpr int t = T, n = N, wt = WT, wn = WN, stages = STAGES;
   static constexpr int warps_t = T / WT;
   static constexpr int stage_bytes = (T + N) * GM_K + T * 16;  // tiles, activation scales [4][T]
-  static constexpr size_t smem = (size_t)STAGES * stage_bytes;
+  // running totals of a thread's sums: in registers where there are few, else in shared memory behind the stages
+  static constexpr bool reg_totals = WT * WN <= 16 * 16;
+  static constexpr size_t smem = (size_t)STAGES * stage_bytes + (reg_totals ? 0 : (size_t)T * N * 4);
   static_assert((T / WT) * (N / WN) * 32 == GM_THREADS, "eight warps");
 };
 using GmLarge = GmTile<128, 128, 64, 32, 4>;
@@ -622,7 +627,7 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
   const int nkb = k / BLOCK, nk = (k + GM_K - 1) / GM_K, nsr = (n_out + BLOCK - 1) / BLOCK;
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   // the tile's weight scales [NBW][nkb] as fp32, brought in once: asked for step by step, each step waited for one
-  float* s_w = reinterpret_cast<float*>(smem + (size_t)GM_STAGES * GM_STAGE_BYTES);
+  float* s_w = reinterpret_cast<float*>(smem + TL::smem);
   for (int i = tid; i < NBW * nkb; i += GM_THREADS) {
     const int r = n0 / BLOCK + i / nkb;
     const size_t at = (size_t)min(r, nsr - 1) * nkb + i % nkb;
@@ -650,76 +655,93 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
   };
   const int lr = lane & 7, lm = lane >> 3;  // ldmatrix: this lane's row of matrix lm
   float acc[MA][NC][4];
-  // The two NaN codes of E4M3 read as zero.  A tile runs unmasked first: a NaN weight shows as a NaN in the sums, and
-  // only then the tile is made again with the codes masked.
-  for (int masked = 0; masked < 2; ++masked) {
+  // K is summed in slices: after each the slice goes to the running total, and what that addition rounded off starts the
+  // next slice.  A single running sum over K = 8192 is off by 1.45e-7 of the result's norm; the kernels for fewer tokens,
+  // which split K over warps, by 7e-8 to 9e-8; this one by 4.4e-8 (blocks of 32) and 6.7e-8 (blocks of 128).
+  const int slice = BLOCK == 128 && k >= 4096 ? 8 : 4;  // K steps: the totals in shared memory cost 1000 cycles a slice
+  float tot[TL::reg_totals ? MA : 1][TL::reg_totals ? NC : 1][4];
+  float* s_tot = reinterpret_cast<float*>(smem + (size_t)GM_STAGES * GM_STAGE_BYTES) + tid;  // [MA * NC * 4][threads]
+  auto each = [&](auto&& f) {
 #pragma unroll
     for (int a = 0; a < MA; ++a)
 #pragma unroll
-      for (int b = 0; b < NC; ++b) acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.f;
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if constexpr (TL::reg_totals) f(acc[a][c][i], tot[a][c][i]);
+          else f(acc[a][c][i], s_tot[((a * NC + c) * 4 + i) * GM_THREADS]);
+        }
+  };
+  // The two NaN codes of E4M3 read as zero.  A tile runs unmasked first: a NaN weight shows as a NaN in the sums, and
+  // only then the tile is made again with the codes masked.
+  for (int masked = 0; masked < 2; ++masked) {
+    each([](float& v, float& s) { v = s = 0.f; });
 #pragma unroll
     for (int i = 0; i < GM_STAGES - 1; ++i) {
       if (i < nk) load(i);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    for (int kt = 0; kt < nk; ++kt) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(GM_STAGES - 2) : "memory");
-      __syncthreads();
-      if (kt + GM_STAGES - 1 < nk) load(kt + GM_STAGES - 1);
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      const uint8_t* stp = smem + (kt % GM_STAGES) * GM_STAGE_BYTES;
-      const uint32_t st = sbase + (kt % GM_STAGES) * GM_STAGE_BYTES;
-      const float* s_as = reinterpret_cast<const float*>(stp + (GM_T + GM_N) * GM_K);
+    for (int k0 = 0; k0 < nk; k0 += slice) {
+      for (int kt = k0; kt < min(k0 + slice, nk); ++kt) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GM_STAGES - 2) : "memory");
+        __syncthreads();
+        if (kt + GM_STAGES - 1 < nk) load(kt + GM_STAGES - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const uint8_t* stp = smem + (kt % GM_STAGES) * GM_STAGE_BYTES;
+        const uint32_t st = sbase + (kt % GM_STAGES) * GM_STAGE_BYTES;
+        const float* s_as = reinterpret_cast<const float*>(stp + (GM_T + GM_N) * GM_K);
 #pragma unroll
-      for (int b = 0; b < BPS; ++b) {
-        float d[MA][NC][4];
+        for (int b = 0; b < BPS; ++b) {
+          uint32_t wb[MPB][NC / 2][4];
 #pragma unroll
-        for (int a = 0; a < MA; ++a)
+          for (int m = 0; m < MPB; ++m) {
+            const int ch = (b * MPB + m) * 2;  // first 16-byte chunk of these 32 codes
 #pragma unroll
-          for (int c = 0; c < NC; ++c) d[a][c][0] = d[a][c][1] = d[a][c][2] = d[a][c][3] = 0.f;
+            for (int c = 0; c < NC / 2; ++c) {  // weight rows wn + 16c ..: {rows 0-7, 8-15} x {chunk, chunk + 1}
+              const int r = wn + c * 16 + (lm >> 1) * 8 + lr;
+              gm_ldsm4(wb[m][c], st + GM_T * GM_K + r * GM_K + (((ch + (lm & 1)) ^ (r & 7)) << 4));
+              if (masked) {
 #pragma unroll
-        for (int m = 0; m < MPB; ++m) {
-          const int ch = (b * MPB + m) * 2;  // first 16-byte chunk of these 32 codes
-          uint32_t wb[NC / 2][4];
-#pragma unroll
-          for (int c = 0; c < NC / 2; ++c) {  // weight rows wn + 16c ..: {rows 0-7, 8-15} x {chunk, chunk + 1}
-            const int r = wn + c * 16 + (lm >> 1) * 8 + lr;
-            gm_ldsm4(wb[c], st + GM_T * GM_K + r * GM_K + (((ch + (lm & 1)) ^ (r & 7)) << 4));
-            if (masked) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) wb[c][i] = e4m3x4_nan_to_zero(wb[c][i]);
+                for (int i = 0; i < 4; ++i) wb[m][c][i] = e4m3x4_nan_to_zero(wb[m][c][i]);
+              }
             }
           }
+          if (kt * BPS + b >= nkb) break;  // behind the end of K
+          const float ws = s_w[(BLOCK == 32 ? wn / 32 : 0) * nkb + kt * BPS + b];
 #pragma unroll
           for (int a = 0; a < MA; ++a) {
-            uint32_t xa[4];
-            const int r = wt + a * 16 + (lm & 1) * 8 + lr;
-            gm_ldsm4(xa, st + r * GM_K + (((ch + (lm >> 1)) ^ (r & 7)) << 4));
+            float d[NC][4];
 #pragma unroll
-            for (int c = 0; c < NC; ++c) qmma_e4m3(d[a][c], xa[0], xa[1], xa[2], xa[3], wb[c >> 1][(c & 1) * 2], wb[c >> 1][(c & 1) * 2 + 1]);
-          }
-        }
-        if (kt * BPS + b >= nkb) break;  // behind the end of K
-        const float ws = s_w[(BLOCK == 32 ? wn / 32 : 0) * nkb + kt * BPS + b];
+            for (int c = 0; c < NC; ++c) d[c][0] = d[c][1] = d[c][2] = d[c][3] = 0.f;
 #pragma unroll
-        for (int a = 0; a < MA; ++a) {
-          const float s0 = s_as[b * GM_T + wt + a * 16 + g] * ws, s1 = s_as[b * GM_T + wt + a * 16 + g + 8] * ws;
+            for (int m = 0; m < MPB; ++m) {
+              const int ch = (b * MPB + m) * 2;
+              uint32_t xa[4];
+              const int r = wt + a * 16 + (lm & 1) * 8 + lr;
+              gm_ldsm4(xa, st + r * GM_K + (((ch + (lm >> 1)) ^ (r & 7)) << 4));
 #pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            acc[a][c][0] = fmaf(d[a][c][0], s0, acc[a][c][0]);
-            acc[a][c][1] = fmaf(d[a][c][1], s0, acc[a][c][1]);
-            acc[a][c][2] = fmaf(d[a][c][2], s1, acc[a][c][2]);
-            acc[a][c][3] = fmaf(d[a][c][3], s1, acc[a][c][3]);
+              for (int c = 0; c < NC; ++c) qmma_e4m3(d[c], xa[0], xa[1], xa[2], xa[3], wb[m][c >> 1][(c & 1) * 2], wb[m][c >> 1][(c & 1) * 2 + 1]);
+            }
+            const float s0 = s_as[b * GM_T + wt + a * 16 + g] * ws, s1 = s_as[b * GM_T + wt + a * 16 + g + 8] * ws;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              acc[a][c][0] = fmaf(d[c][0], s0, acc[a][c][0]);
+              acc[a][c][1] = fmaf(d[c][1], s0, acc[a][c][1]);
+              acc[a][c][2] = fmaf(d[c][2], s1, acc[a][c][2]);
+              acc[a][c][3] = fmaf(d[c][3], s1, acc[a][c][3]);
+            }
           }
         }
       }
+      each([](float& v, float& s) {
+        const float n = s + v;
+        v = fabsf(n) <= FLT_MAX ? v - (n - s) : 0.f;  // an infinite sum has no remainder
+        s = n;
+      });
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     float chk = 0.f;
-#pragma unroll
-    for (int a = 0; a < MA; ++a)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) chk += (acc[a][c][0] + acc[a][c][1]) + (acc[a][c][2] + acc[a][c][3]);
+    each([&](float& v, float& s) { chk += v += s; });
     if (!__syncthreads_or(chk != chk)) break;
   }
 #pragma unroll
@@ -747,8 +769,8 @@ static cudaError_t launch_gemm(int block, cudaStream_t s, const uint8_t* codes, 
   auto go = [&](auto kern, auto tile) {
     using TL = decltype(tile);
     const dim3 grid((rows + TL::t - 1) / TL::t, (n + TL::n - 1) / TL::n);
-    const size_t smem = TL::smem + (size_t)((TL::n + block - 1) / block) * (k / block) * 4;
-    const cudaError_t e = smem_optin_once(kern, 227 * 1024);
+    const size_t smem = TL::smem + gm_scale_bytes(TL::n, k, block);
+    const cudaError_t e = smem_optin_once(kern, GM_SMEM_LIMIT);
     if (e == cudaSuccess) kern<<<grid, GM_THREADS, smem, s>>>(codes, act_scales, weight, w_scales, scale_rule, rows, n, k, out, ldo, addend);
     return e;
   };
@@ -756,7 +778,9 @@ static cudaError_t launch_gemm(int block, cudaStream_t s, const uint8_t* codes, 
     using TL = decltype(tile);
     return block == 32 ? go(fp8_gemm_kernel<32, OutT, TL>, tile) : go(fp8_gemm_kernel<128, OutT, TL>, tile);
   };
-  return rows <= 32 ? pick(GmSmall()) : rows <= 64 ? pick(GmMid()) : pick(GmLarge());
+  if (rows <= 32) return pick(GmSmall());
+  // the large tile while its stages, totals and weight scales fit
+  return rows <= 64 || GmLarge::smem + gm_scale_bytes(GmLarge::n, k, block) > GM_SMEM_LIMIT ? pick(GmMid()) : pick(GmLarge());
 }
 
 // pdl: the kernel directly before this call in the stream is one of this file's quantisers (it writes the codes and

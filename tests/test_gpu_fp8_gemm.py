@@ -32,3 +32,52 @@ def test_rows_match_single_tokens(n, k, rule, rows, nan):
     # bf16 results: the fp32 ones rounded, one step apart where the sum order moved a value over a boundary
     b = cb.fp8_linear(x, w, s).float()
     assert bool(((b - got).abs() <= got.abs() * 2.0 ** -8 + 1e-30).all())
+
+
+@pytest.mark.parametrize("rule", ["e8m0", "f32"])
+@pytest.mark.parametrize("k", [1536, 8192])
+@pytest.mark.parametrize("rows", [32, 64, 300])
+def test_fp32_sums_as_accurate_as_few_tokens(rule, k, rows):
+    """The error of the fp32 results against float64 over 2**13 outputs and more is no larger than that of the streaming GEMV
+    (eight tokens at a time), which adds K in slices; a single running sum over K = 8192 has twice its error."""
+    import torch
+
+    import cachalot_b200 as cb
+
+    n, block = 256, 32 if rule == "e8m0" else 128
+    g = torch.Generator(device="cuda").manual_seed(k + rows)
+    w = (torch.randn((n, k), device="cuda", generator=g) * 64).to(torch.float8_e4m3fn).view(torch.uint8)
+    if rule == "e8m0":
+        s = torch.randint(112, 118, (n // 32, k // 32), device="cuda", generator=g).to(torch.uint8)
+        s64 = torch.ldexp(torch.ones(s.shape, device="cuda", dtype=torch.float64), s.double() - 127)
+    else:
+        s = (torch.rand((n // 128, k // 128), device="cuda", generator=g) + 0.5) * 1e-3
+        s64 = s.double()
+    x = torch.randn((rows, k), device="cuda", generator=g).to(torch.bfloat16)
+    q = cb.quantize_fp8_activation(x, block, rule)
+    x64 = q.values.view(torch.float8_e4m3fn).double() * q.scales.double().repeat_interleave(block, 1)
+    want = x64 @ (w.view(torch.float8_e4m3fn).double() * s64.repeat_interleave(block, 0).repeat_interleave(block, 1)).T
+    err = lambda y: float((y.double() - want).norm() / want.norm())  # noqa: E731
+    many = err(cb.fp8_linear(x, w, s, out_dtype=torch.float32))
+    few = err(torch.cat([cb.fp8_linear(x[i:i + 8], w, s, out_dtype=torch.float32) for i in range(0, rows, 8)]))
+    assert many <= 1.05 * few, f"{many:.3e} against {few:.3e}"  # the figure itself spreads by about 1 % over 8192 outputs
+
+
+@pytest.mark.parametrize("rows", [17, 300])
+def test_infinite_activations(rows):
+    """An infinite activation makes its row's results infinite or NaN exactly where one token at a time makes them so."""
+    import torch
+
+    import cachalot_b200 as cb
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    w = (torch.randn((200, 1024), device="cuda", generator=g) * 64).to(torch.float8_e4m3fn).view(torch.uint8)
+    s = torch.rand((2, 8), device="cuda", generator=g) * 1e-3 + 1e-4
+    x = torch.randn((rows, 1024), device="cuda", generator=g).to(torch.bfloat16)
+    x[1, 3], x[rows - 1, 1000] = float("inf"), float("-inf")
+    got = cb.fp8_linear(x, w, s, out_dtype=torch.float32)
+    want = torch.cat([cb.fp8_linear(x[i:i + 1], w, s, out_dtype=torch.float32) for i in range(rows)])
+    assert bool((torch.isinf(want[1]) | torch.isnan(want[1])).any())
+    bad = ~torch.isfinite(want)
+    assert torch.equal(~torch.isfinite(got), bad)
+    assert torch.equal(torch.nan_to_num(got[bad], nan=7.0), torch.nan_to_num(want[bad], nan=7.0))
