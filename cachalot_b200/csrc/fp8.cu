@@ -580,9 +580,8 @@ extern "C" int cachalot_fp8_act_quant(const void* x_bf16, int rows, int k, int b
 // codes of K sixteen MMAs next to 64 FMAs that apply the scales and six ldmatrix, so issue slots before the tensor pipe.
 // The 64-token kernel above reads every weight again per 64 tokens, straight from L2 into registers: shared expert of
 // 1000 tokens, 5120 x 2304, 2729 us there, 426 us here.
-// Nine to 64 tokens are bound by the weights' way in: small tiles (32 tokens x 64 outputs, or 64 x 32; warps of 16 x 16)
-// that spread a 4096-row matrix over the SMs, two CTAs each, with six stages in flight:
-// 32 tokens through [12288,4096] + [4096,8192] take 81.9 us on the per-lane kernel, 75.8 here.
+// Few tokens are bound by the weights' way in: small tiles (32 tokens x 64 outputs, warps of 16 x 16) with six stages in
+// flight, two CTAs per SM.
 constexpr int GM_K = 128, GM_THREADS = 256, GM_SMEM_LIMIT = 227 * 1024;
 // a tile's weight scales as fp32: [scale rows of the tile][K / block]
 static size_t gm_scale_bytes(int n, int k, int block) { return (size_t)((n + block - 1) / block) * (k / block) * 4; }
@@ -597,7 +596,6 @@ struct GmTile {
   static_assert((T / WT) * (N / WN) * 32 == GM_THREADS, "eight warps");
 };
 using GmLarge = GmTile<128, 128, 64, 32, 4>;
-using GmMid = GmTile<64, 32, 16, 16, 6>;
 using GmSmall = GmTile<32, 64, 16, 16, 6>;
 
 __device__ __forceinline__ void gm_cp16(uint32_t dst, const void* src, int bytes) {
@@ -763,6 +761,29 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
     }
 }
 
+static int gm_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+  return sms;
+}
+
+// The GEMM or the per-lane kernel.  A CTA of the GEMM walks all of K, the per-lane kernel splits it over its warps: up to 16
+// tokens the latter is the faster one for every matrix, up to 32 while its CTAs of 32 rows are one per SM.
+// us per-lane / GEMM, 16 tokens: [1024,8192] 16 / 48, [4096,4096] 17 / 26, [8192,4096] 27 / 27, [12288,4096] 30 / 39;
+// 32 tokens: [1024,8192] 36 / 49, [4608,4096] 23 / 27, [5120,4096] 35 / 27, [12288,4096] 54 / 38.
+static bool gm_takes(int rows, int n) { return rows > 32 || (rows > 16 && (n + 31) / 32 > gm_sms()); }
+
+// The tile, by the rounds its CTAs take on this GPU's SMs (two small ones fit on an SM): a round of large tiles takes 2.5 to 3
+// times one of small tiles, so small ones while they need fewer than 8/3 of the large ones' rounds.  us small / large:
+// [2304,5120] 65 tokens 34 / 120, 256: 54 / 130, 384: 83 / 133; [5120,2304] 65: 25 / 58, 192: 45 / 62, 256: 56 / 62,
+// 384: 77 / 64.
+static bool gm_small(int rows, int n, int k, int block) {
+  if (GmLarge::smem + gm_scale_bytes(GmLarge::n, k, block) > GM_SMEM_LIMIT) return true;
+  const long long sms = gm_sms();
+  auto rounds = [](int rows_, int t, int n_, int w, long long slots) { return ((long long)((rows_ + t - 1) / t) * ((n_ + w - 1) / w) + slots - 1) / slots; };
+  return 3 * rounds(rows, GmSmall::t, n, GmSmall::n, 2 * sms) <= 8 * rounds(rows, GmLarge::t, n, GmLarge::n, sms);
+}
+
 template <typename OutT>
 static cudaError_t launch_gemm(int block, cudaStream_t s, const uint8_t* codes, const float* act_scales, const uint8_t* weight,
                                const void* w_scales, int scale_rule, int rows, int n, int k, OutT* out, long long ldo, const float* addend) {
@@ -778,9 +799,7 @@ static cudaError_t launch_gemm(int block, cudaStream_t s, const uint8_t* codes, 
     using TL = decltype(tile);
     return block == 32 ? go(fp8_gemm_kernel<32, OutT, TL>, tile) : go(fp8_gemm_kernel<128, OutT, TL>, tile);
   };
-  if (rows <= 32) return pick(GmSmall());
-  // the large tile while its stages, totals and weight scales fit
-  return rows <= 64 || GmLarge::smem + gm_scale_bytes(GmLarge::n, k, block) > GM_SMEM_LIMIT ? pick(GmMid()) : pick(GmLarge());
+  return gm_small(rows, n, k, block) ? pick(GmSmall()) : pick(GmLarge());
 }
 
 // pdl: the kernel directly before this call in the stream is one of this file's quantisers (it writes the codes and
@@ -796,15 +815,15 @@ static int gemv_checked(const char* who, const uint8_t* codes, const float* act_
   if (!aligned(weight, 8) || !aligned(codes, 8) || k % 8) return fail(CACHALOT_EALIGN, "%s: weight and codes need 8-byte alignment", who);
   if (ldo < n) return fail(CACHALOT_EINVAL, "%s: output row pitch %lld < %d", who, ldo, n);
   if (rows == 0) return CACHALOT_OK;
-  // More than eight tokens: the tiled GEMM (its 16-byte copies need 16-byte rows; K is bounded by the room for scales)
-  if (rows > 8 && aligned(weight, 16) && aligned(codes, 16) && k % 16 == 0 && n <= 32 * 65535 && k <= 1 << 16) {
+  // the tiled GEMM (its 16-byte copies need 16-byte rows; K is bounded by the room for scales)
+  if (gm_takes(rows, n) && aligned(weight, 16) && aligned(codes, 16) && k % 16 == 0 && n <= 32 * 65535 && k <= 1 << 16) {
     const cudaError_t e = out_dtype == CACHALOT_BF16
                               ? launch_gemm(block, s, codes, act_scales, weight, w_scales, scale_rule, rows, n, k, (__nv_bfloat16*)out, ldo, addend)
                               : launch_gemm(block, s, codes, act_scales, weight, w_scales, scale_rule, rows, n, k, (float*)out, ldo, addend);
     if (e != cudaSuccess) return fail(CACHALOT_ECUDA, "%s: %s", who, cudaGetErrorString(e));
     return check_launch(who);
   }
-  // 64 tokens per launch; more tokens (of rows that are not 16-byte aligned) take more launches over the same weights
+  // 64 tokens per launch; more of them (rows that are not 16-byte aligned) take more launches over the same weights
   for (int r0 = 0; r0 < rows; r0 += 8 * GEMV_MAX_TG) {
     const int nr = rows - r0 < 8 * GEMV_MAX_TG ? rows - r0 : 8 * GEMV_MAX_TG;
     const int ntg = (nr + 7) / 8;
@@ -814,8 +833,8 @@ static int gemv_checked(const char* who, const uint8_t* codes, const float* act_
     static const bool no_stream = [] { const char* e = std::getenv("CACHALOT_FP8_PER_LANE"); return e && e[0] == '1'; }();
     GsGeo G;
     bool staged = false;
-    // up to eight tokens; beyond that the activation fragments outweigh the weights and the per-lane kernel, which
-    // shares them between two row tiles, is the faster one of the two (rows that the GEMM does not take)
+    // up to eight tokens; beyond that the activation fragments outweigh the weights and the per-lane kernel is the faster
+    // one of the two (from 17 tokens it shares them between two row tiles)
     if (!no_stream && ntg == 1 && gs_geometry(nr, k, block, 1, &staged, &G)) {
       cudaError_t e;
       if (out_dtype == CACHALOT_BF16) {

@@ -1,4 +1,4 @@
-"""The tiled FP8 GEMM (more than eight tokens) against the streaming GEMV (one token at a time, itself checked against the oracle):
+"""FP8 linears of more than eight tokens against the streaming GEMV (one token at a time, itself checked against the oracle):
 the same products summed in fp32 in another order, at sizes that end inside a tile, a K step and a scale block row; weights
 that hold the two NaN codes, which read as zero."""
 import pytest
@@ -81,3 +81,35 @@ def test_infinite_activations(rows):
     bad = ~torch.isfinite(want)
     assert torch.equal(~torch.isfinite(got), bad)
     assert torch.equal(torch.nan_to_num(got[bad], nan=7.0), torch.nan_to_num(want[bad], nan=7.0))
+
+
+@pytest.mark.parametrize("rows,n,k,per_lane", [(9, 4096, 1024, True), (16, 4096, 1024, True), (32, 1024, 1024, True), (32, 4736, 512, True),
+                                               (17, 4800, 512, False), (33, 200, 416, False), (80, 200, 416, False), (300, 130, 1024, False)])
+@pytest.mark.parametrize("rule", ["e8m0", "f32"])
+def test_weights_off_sixteen_bytes(rows, n, k, per_lane, rule):
+    """Rows that are not 16-byte aligned always take the kernel that splits K over warps.  Up to 16 tokens, and up to 32 of a
+    matrix whose 32-row CTAs fit on the SMs at once, aligned rows take it too (the GEMM needs up to three times as long
+    there): the same bits.  Other calls differ by the order of the fp32 sums."""
+    import torch
+
+    import cachalot_b200 as cb
+
+    if rule == "f32" and k % 128:
+        pytest.skip("blocks of 128")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert per_lane == (rows <= 16 or (rows <= 32 and -(-n // 32) <= sms)), "the sizes are chosen for 148 SMs"
+    g = torch.Generator(device="cuda").manual_seed(n + k + rows)
+    w = (torch.randn((n, k), device="cuda", generator=g) * 64).to(torch.float8_e4m3fn).view(torch.uint8)
+    off = torch.empty(n * k + 8, dtype=torch.uint8, device="cuda")[8:].view(n, k)
+    off.copy_(w)
+    assert w.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 8
+    if rule == "e8m0":
+        s = torch.randint(112, 118, (-(-n // 32), k // 32), device="cuda", generator=g).to(torch.uint8)
+    else:
+        s = (torch.rand((-(-n // 128), k // 128), device="cuda", generator=g) + 0.1) * 1e-3
+    x = torch.randn((rows, k), device="cuda", generator=g).to(torch.bfloat16)
+    a, b = cb.fp8_linear(x, w, s, out_dtype=torch.float32), cb.fp8_linear(x, off, s, out_dtype=torch.float32)
+    if per_lane:
+        assert torch.equal(a, b)
+    else:  # as in test_rows_match_single_tokens
+        assert bool(((a - b).abs() <= 4 * k * 2.0 ** -24 * b.abs().amax(1, keepdim=True)).all())
