@@ -656,7 +656,9 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
   // K is summed in slices: after each the slice goes to the running total, and what that addition rounded off starts the
   // next slice.  A single running sum over K = 8192 is off by 1.45e-7 of the result's norm; the kernels for fewer tokens,
   // which split K over warps, by 7e-8 to 9e-8; this one by 4.4e-8 (blocks of 32) and 6.7e-8 (blocks of 128).
-  const int slice = BLOCK == 128 && k >= 4096 ? 8 : 4;  // K steps: the totals in shared memory cost 1000 cycles a slice
+  // Steps of K per slice: as few as keep the error at short K below that of those kernels, too; adding a slice to the totals
+  // in shared memory costs 1000 cycles.
+  const int slice = BLOCK == 32 ? min((nk + 3) / 4, 4) : min(max((nk + 2) / 3, 4), 8);
   float tot[TL::reg_totals ? MA : 1][TL::reg_totals ? NC : 1][4];
   float* s_tot = reinterpret_cast<float*>(smem + (size_t)GM_STAGES * GM_STAGE_BYTES) + tid;  // [MA * NC * 4][threads]
   auto each = [&](auto&& f) {
@@ -673,7 +675,7 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
   // The two NaN codes of E4M3 read as zero.  A tile runs unmasked first: a NaN weight shows as a NaN in the sums, and
   // only then the tile is made again with the codes masked.
   for (int masked = 0; masked < 2; ++masked) {
-    each([](float& v, float& s) { v = s = 0.f; });
+    each([](float& v, float&) { v = 0.f; });
 #pragma unroll
     for (int i = 0; i < GM_STAGES - 1; ++i) {
       if (i < nk) load(i);
@@ -690,21 +692,8 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
         const float* s_as = reinterpret_cast<const float*>(stp + (GM_T + GM_N) * GM_K);
 #pragma unroll
         for (int b = 0; b < BPS; ++b) {
-          uint32_t wb[MPB][NC / 2][4];
-#pragma unroll
-          for (int m = 0; m < MPB; ++m) {
-            const int ch = (b * MPB + m) * 2;  // first 16-byte chunk of these 32 codes
-#pragma unroll
-            for (int c = 0; c < NC / 2; ++c) {  // weight rows wn + 16c ..: {rows 0-7, 8-15} x {chunk, chunk + 1}
-              const int r = wn + c * 16 + (lm >> 1) * 8 + lr;
-              gm_ldsm4(wb[m][c], st + GM_T * GM_K + r * GM_K + (((ch + (lm & 1)) ^ (r & 7)) << 4));
-              if (masked) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) wb[m][c][i] = e4m3x4_nan_to_zero(wb[m][c][i]);
-              }
-            }
-          }
           if (kt * BPS + b >= nkb) break;  // behind the end of K
+          uint32_t wb[MPB][NC / 2][4];  // the block's weights, loaded for the first row tile
           const float ws = s_w[(BLOCK == 32 ? wn / 32 : 0) * nkb + kt * BPS + b];
 #pragma unroll
           for (int a = 0; a < MA; ++a) {
@@ -713,7 +702,18 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
             for (int c = 0; c < NC; ++c) d[c][0] = d[c][1] = d[c][2] = d[c][3] = 0.f;
 #pragma unroll
             for (int m = 0; m < MPB; ++m) {
-              const int ch = (b * MPB + m) * 2;
+              const int ch = (b * MPB + m) * 2;  // first 16-byte chunk of these 32 codes
+              if (a == 0) {
+#pragma unroll
+                for (int c = 0; c < NC / 2; ++c) {  // weight rows wn + 16c ..: {rows 0-7, 8-15} x {chunk, chunk + 1}
+                  const int r = wn + c * 16 + (lm >> 1) * 8 + lr;
+                  gm_ldsm4(wb[m][c], st + GM_T * GM_K + r * GM_K + (((ch + (lm & 1)) ^ (r & 7)) << 4));
+                  if (masked) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) wb[m][c][i] = e4m3x4_nan_to_zero(wb[m][c][i]);
+                  }
+                }
+              }
               uint32_t xa[4];
               const int r = wt + a * 16 + (lm & 1) * 8 + lr;
               gm_ldsm4(xa, st + r * GM_K + (((ch + (lm >> 1)) ^ (r & 7)) << 4));
@@ -731,15 +731,21 @@ fp8_gemm_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ act
           }
         }
       }
-      each([](float& v, float& s) {
-        const float n = s + v;
-        v = fabsf(n) <= FLT_MAX ? v - (n - s) : 0.f;  // an infinite sum has no remainder
-        s = n;
-      });
+      if (k0 + slice >= nk) {
+        if (k0) each([](float& v, float& s) { v += s; });
+      } else if (k0 == 0) {
+        each([](float& v, float& s) { s = v, v = 0.f; });
+      } else {
+        each([](float& v, float& s) {
+          const float n = s + v;
+          v = fabsf(n) <= FLT_MAX ? v - (n - s) : 0.f;  // an infinite sum has no remainder
+          s = n;
+        });
+      }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     float chk = 0.f;
-    each([&](float& v, float& s) { chk += v += s; });
+    each([&](float& v, float&) { chk += v; });
     if (!__syncthreads_or(chk != chk)) break;
   }
 #pragma unroll
