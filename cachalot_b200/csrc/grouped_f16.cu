@@ -422,9 +422,13 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
   }
 }
 
+__device__ __forceinline__ float finite_or_0(float v) { return fabsf(v) <= 3.4e38f ? v : 0.f; }
+
 // One CTA per grouped row: bf16 row src[p] (or p) of [., k] -> fp16 row p times a power of two, codes j and j+8 of every
 // sixteen side by side, behind it the sums of its blocks (twice: against the biases and the scales) as high and low
-// halves.  out fp16 [rows, pitch], row_scale f32 [rows] = the inverse of the power of two.
+// halves.  out fp16 [rows, pitch], row_scale f32 [rows] = the inverse of the power of two.  An infinite or NaN value shows in
+// its block's sum alone, against the bias alone, so that the product is bias * sum as in the one-token kernel: as an
+// operand of its own it would meet zeros and both signs of s*(q-1).
 __global__ void prep_rows_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ src, KShape K, __half* __restrict__ out,
                                  float* __restrict__ row_scale) {
   __shared__ float part[32];
@@ -438,14 +442,14 @@ __global__ void prep_rows_kernel(const __nv_bfloat16* __restrict__ x, const int3
     const uint32_t wds[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(wds[j] << 16)), fabsf(__uint_as_float(wds[j] & 0xffff0000u))));
+      amax = fmaxf(amax, fmaxf(fabsf(finite_or_0(__uint_as_float(wds[j] << 16))), fabsf(finite_or_0(__uint_as_float(wds[j] & 0xffff0000u)))));
   }
   amax = warp_max(amax);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = amax;
   __syncthreads();
   amax = warp_max((threadIdx.x & 31) < (blockDim.x >> 5) ? part[threadIdx.x & 31] : 0.f);
   const int eb = (int)(__float_as_uint(amax) >> 23);
-  const int e = (eb == 0 || eb == 255) ? 0 : min(134 - eb, 126);  // largest value into [2^7, 2^8); zeros and infinities as they are
+  const int e = eb == 0 ? 0 : min(134 - eb, 126);  // largest finite value into [2^7, 2^8); a row of zeros as it is
   const float sc = pow2f(e);
   if (threadIdx.x == 0) row_scale[p] = pow2f(-e);
   const int per = K.block / 16;  // sixteens per block: 4 or 8 neighbouring threads
@@ -459,8 +463,10 @@ __global__ void prep_rows_kernel(const __nv_bfloat16* __restrict__ x, const int3
       __half h[16];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        h[2 * j] = __float2half_rn(__uint_as_float(wds[j] << 16) * sc);
-        h[2 * j + 1] = __float2half_rn(__uint_as_float(wds[j] & 0xffff0000u) * sc);
+        const float a = __uint_as_float(wds[j] << 16), b = __uint_as_float(wds[j] & 0xffff0000u);
+        h[2 * j] = __float2half_rn(finite_or_0(a) * sc);
+        h[2 * j + 1] = __float2half_rn(finite_or_0(b) * sc);
+        sum += (a - finite_or_0(a)) + (b - finite_or_0(b));  // 0 where both are finite
       }
       __half2 r[8];
 #pragma unroll
@@ -474,9 +480,10 @@ __global__ void prep_rows_kernel(const __nv_bfloat16* __restrict__ x, const int3
     for (int d = 1; d < per; d <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
     if (g < n16 && g % per == 0) {
       const int j = g / per;
-      const __half hi = __float2half_rn(sum), lo = __float2half_rn(sum - __half2float(hi));
+      const bool fin = fabsf(sum) <= 65504.f;
+      const __half hi = __float2half_rn(sum), lo = __float2half_rn(fin ? sum - __half2float(hi) : 0.f);
       __half* e0 = o + K.k + j;
-      e0[0] = e0[K.n_block] = hi;
+      e0[0] = hi, e0[K.n_block] = fin ? hi : __float2half_rn(0.f);
       e0[K.ext] = e0[K.ext + K.n_block] = lo;
     }
   }

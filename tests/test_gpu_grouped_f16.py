@@ -84,6 +84,31 @@ def test_stages_with_one_operand_slot(hidden, inter, group):
     assert within_bf16_flips(got[some].cpu().numpy(), _want(x[some], slots[some], w[some], experts, group))
 
 
+def test_infinite_and_nan_activations():
+    """An infinite or NaN activation does to its row, and to no other, what it does in the one-token kernel.  All biases of
+    these banks are negative: -inf drives gate and up to +inf, which the clamp makes finite again, as it does NaN; +inf ends
+    as NaN."""
+    import torch
+
+    import cachalot_b200 as cb
+
+    rng = np.random.default_rng(11)
+    experts, bank = _bank(rng, 512, 320, 3, 128)
+    assert all((e[f"{p}.biases"] < 0).all() for e in experts for p in ("w1", "w3"))
+    x = rng.standard_normal((24, 512)).astype(np.float32)
+    x[1, 70], x[2, 511], x[3, 0], x[4, [3, 300]], x[5] = -np.inf, np.inf, np.nan, -np.inf, x[5] * 1e30
+    xt = bf16_tensor(x)
+    slots = torch.from_numpy(np.stack([rng.permutation(3)[:2] for _ in range(24)]).astype(np.int32)).cuda()
+    w = torch.rand((24, 2), device="cuda") + 0.1
+    got = cb.moe_forward(xt, slots, w, bank).cpu().numpy()
+    want = torch.cat([cb.moe_forward(xt[i:i + 1], slots[i:i + 1], w[i:i + 1], bank) for i in range(24)]).cpu().numpy()
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.isnan(want[2]).all() and np.isfinite(want[[0, 1, 3, 4, 5]]).all()
+    for t in (1, 3, 4, 5):  # every expert's output is one bf16 rounding away from the other kernel's, at most one step
+        assert np.abs(got[t] - want[t]).max() < 2.0 ** -7 * np.abs(want[t]).max(), f"token {t}"
+    xt[1:6] = 1.0
+    assert np.array_equal(cb.moe_forward(xt, slots, w, bank).cpu().numpy()[6:], got[6:])
+
+
 def test_more_rows_than_one_plan():
     import torch
 
