@@ -598,15 +598,20 @@ bool f16_supported(const BankView& v) {
          stages(1, windows(v.inter, v.group)) >= 2;
 }
 
-size_t decode_f16_workspace_bytes(const BankView& v, int rows, int k) {
-  return carve_f16(nullptr, v, (size_t)min(rows, PLAN_ROWS_MAX / k) * k, 0).total;
+// as few runs of whole tokens as the planning kernel's limit allows, as equal as they can be
+int decode_f16_run(int rows, int k) {
+  const int most = max(PLAN_ROWS_MAX / k, 1), runs = (rows + most - 1) / most;
+  return (rows + runs - 1) / runs;
 }
 
-// Routed experts of a decode batch, reference rounding points; more routed rows than the planning kernel takes go in
-// runs of whole tokens.
+size_t decode_f16_workspace_bytes(const BankView& v, int rows, int k) {
+  return carve_f16(nullptr, v, (size_t)decode_f16_run(rows, k) * k, 0).total;
+}
+
+// Routed experts of a decode batch, reference rounding points, run by run.
 int launch_decode_f16(const BankView& v, const void* x_bf16, const int32_t* slots, const float* gate_w, int rows, int k, float limit,
                       void* workspace, void* out, int out_dtype, int* status, cudaStream_t stream) {
-  const int chunk = min(rows, PLAN_ROWS_MAX / k);
+  const int chunk = decode_f16_run(rows, k);
   const F16Scratch s = carve_f16(static_cast<uint8_t*>(workspace), v, (size_t)chunk * k, 0);
   for (int r0 = 0; r0 < rows; r0 += chunk) {
     const int n = min(chunk, rows - r0), R = n * k;

@@ -102,6 +102,7 @@ bool decode_tc_supported(const BankView& v, int rows, int k);
 // Several tokens over the 2-bit bank (fp16 scales, the reference's bf16 rounding points) on the f16 tensor cores, every
 // distinct expert streamed once (grouped_f16.cu).
 bool f16_supported(const BankView& v);
+int decode_f16_run(int rows, int k);  // tokens of one run of a decode batch
 size_t decode_f16_workspace_bytes(const BankView& v, int rows, int k);
 int launch_decode_f16(const BankView& v, const void* x_bf16, const int32_t* slots, const float* gate_w, int rows, int k, float limit,
                       void* workspace, void* out, int out_dtype, int* status, cudaStream_t stream);

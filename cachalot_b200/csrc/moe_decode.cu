@@ -286,16 +286,30 @@ static int grouped_tc_min_rows() {  // CACHALOT_GROUPED_MIN_ROWS overrides the b
   return v;
 }
 #define GROUPED_TC_MIN_ROWS grouped_tc_min_rows()
-// 2-bit bank with fp16 scales, reference rounding points: the grouped f16 kernels pay per distinct expert (about 11 us at
-// 4096 x 2880: unpacking its codes), the per-token kernel per routed row (3.8 us), so the former take the call when the
-// rows are at least three times the experts there can be.
-static bool grouped_f16_pays(long long routed_rows, long long n_experts) { return routed_rows >= 3 * n_experts; }
+// 2-bit bank with fp16 scales, reference rounding points: do the grouped f16 kernels beat the one-token kernel?  Both sides
+// in us, fitted to 480 timings (2048 x 768 to 5120 x 2304, 1 to 384 experts, 3 to 1024 routed rows of one or six per token,
+// uniform and Zipf routing).  The grouped kernels take 30 + 5.5 per 1000 of hidden + inter for their launches and one
+// unit's walk over K, and unpack every unit of up to 64 rows of one expert: 0.4 + 0.68 per million weights of a matrix.
+// A token takes 10.5 and 0.205 per routed expert and million weights.  The experts are counted as the most the rows can
+// touch, so a call whose rows share fewer may stay with the one-token kernel although the grouped ones would be faster;
+// none of the 480 took the slower route.  4096 x 2880, 6 per token, us grouped / one-token: 16 experts, 48 rows 206 / 194,
+// 96: 210 / 378; 128 experts, 258 rows 972 / 996, 384: 1119 / 1476; 384 experts, 384 rows 2075 / 1475, 768: 2848 / 2928.
+static bool grouped_f16_pays(const BankView& v, long long tokens, int k, long long n_experts) {
+  const double weights = 1e-6 * v.hidden * v.inter, rows = (double)tokens * k;
+  const double units = std::min(rows, (double)n_experts) + std::floor(rows / 64);
+  return 30 + 5.5e-3 * (v.hidden + v.inter) + units * (0.4 + 0.68 * weights) < tokens * (10.5 + 0.205 * k * weights);
+}
 
 // the descriptor's fields that f16_supported() and its scratch sizes look at
 static BankView shape_view(const cachalot_bank_desc* d) {
   BankView v = {};
   v.format = d->format, v.bits = d->bits, v.group = d->group, v.scale_dtype = d->scale_dtype, v.hidden = d->hidden, v.inter = d->inter;
   return v;
+}
+
+// a batch goes in runs of equal length, each of which unpacks its experts anew: the rule is asked for one of them
+static bool decode_f16_takes(const BankView& v, int rows, int k, int n_slots) {
+  return f16_supported(v) && grouped_f16_pays(v, decode_f16_run(rows, k), k, n_slots);
 }
 
 // what moe_decode cannot do without; with less than cachalot_moe_decode_workspace_bytes a 2-bit bank goes token by token
@@ -313,7 +327,7 @@ extern "C" size_t cachalot_moe_decode_workspace_bytes(const cachalot_bank_desc* 
   if (!desc || rows <= 0 || k <= 0) return 0;
   const size_t m = decode_min_workspace(desc, rows, k);
   const BankView v = shape_view(desc);
-  const size_t f = f16_supported(v) && grouped_f16_pays((long long)rows * k, desc->n_slots) && k <= 64 ? decode_f16_workspace_bytes(v, rows, k) : 0;
+  const size_t f = k <= 64 && decode_f16_takes(v, rows, k, desc->n_slots) ? decode_f16_workspace_bytes(v, rows, k) : 0;
   return m > f ? m : f;
 }
 
@@ -341,7 +355,7 @@ extern "C" int cachalot_moe_decode(const void* bank, const cachalot_bank_desc* d
       ((numerics & 0xff) == CACHALOT_NUMERICS_F32 || (numerics & 0xff) == CACHALOT_NUMERICS_BF16))
     return launch_decode_tc(v, x_bf16, slots, gate_w, rows, k, swiglu_limit, workspace, out, out_dtype, status, (cudaStream_t)stream,
                             (numerics & 0xff) == CACHALOT_NUMERICS_BF16);
-  if (fused_ok && f16_supported(v) && grouped_f16_pays((long long)rows * k, v.n_slots) && (numerics & 0xff) == CACHALOT_NUMERICS_BF16 &&
+  if (fused_ok && decode_f16_takes(v, rows, k, v.n_slots) && (numerics & 0xff) == CACHALOT_NUMERICS_BF16 &&
       workspace_bytes >= decode_f16_workspace_bytes(v, rows, k))
     return launch_decode_f16(v, x_bf16, slots, gate_w, rows, k, swiglu_limit, workspace, out, out_dtype, status, (cudaStream_t)stream);
   // Up to 64 tokens: one single-launch kernel per token, back to back.  Tokens share few experts at these sizes (384
@@ -372,7 +386,7 @@ extern "C" int cachalot_moe_decode(const void* bank, const cachalot_bank_desc* d
 
 extern "C" size_t cachalot_moe_layer_decode_workspace_bytes(const cachalot_bank_desc* desc, int k) {
   if (!desc || k <= 0) return 0;
-  return cachalot_moe_decode_workspace_bytes(desc, 1, k) + 1024;  // + indices, weights, slots of the two-call path
+  return decode_min_workspace(desc, 1, k) + 1024;  // + indices, weights, slots of the two-call path
 }
 
 extern "C" int cachalot_moe_layer_decode(const void* bank, const cachalot_bank_desc* desc, const void* x_bf16,
@@ -526,7 +540,7 @@ extern "C" int cachalot_moe_prefill(const void* bank, const cachalot_bank_desc* 
   if (tc)
     return launch_prefill_tc(v, x_bf16, perm, offsets, slot_of_expert, gate_w, tokens, k, n_experts, swiglu_limit, workspace, out,
                              status, s);
-  if (!mxfp4_act && f16_supported(v) && n_experts <= 8192 && grouped_f16_pays(rows, n_experts) &&
+  if (!mxfp4_act && f16_supported(v) && n_experts <= 8192 && grouped_f16_pays(v, tokens, k, n_experts) &&
       workspace_bytes >= prefill_f16_workspace_bytes(v, tokens, k, n_experts))
     return launch_prefill_f16(v, x_bf16, perm, offsets, slot_of_expert, gate_w, tokens, k, n_experts, swiglu_limit, workspace, out, status, s);
   uint8_t* ws = static_cast<uint8_t*>(workspace);

@@ -79,3 +79,25 @@ def test_bank_layout_and_sizes():
     aff = tensor_sizes(affine_format(4096, 2880), 4096, 2880)
     assert sum(aff.values()) == 9_953_280
     assert sum(tensor_sizes(FP4_FORMAT, 5120, 2304).values()) == 18_800_640
+
+
+def _affine_desc(hidden, inter, n_slots):
+    from cachalot_b200 import _lib
+    from cachalot_b200.bank import affine_format, tensor_sizes
+
+    d = _lib.BankDesc()
+    sizes = list(tensor_sizes(affine_format(hidden, inter), hidden, inter).values())
+    at = 0
+    for i, s in enumerate(sizes):
+        d.off[i], at = at, at + -(-s // 256) * 256
+    d.record_bytes, d.n_slots, d.hidden, d.inter = at, n_slots, hidden, inter
+    d.format, d.bits, d.group, d.scale_dtype = _lib.BANK_AFFINE, 2, 128, _lib.F16
+    return d
+
+
+def test_one_token_scratch_does_not_depend_on_the_slots():
+    from cachalot_b200 import _lib
+
+    size = lambda slots, k: _lib.lib.cachalot_moe_layer_decode_workspace_bytes(ctypes.byref(_affine_desc(4096, 2880, slots)), k)  # noqa: E731
+    for k in (1, 6, 32):
+        assert size(1, k) == size(2, k) == size(384, k)
