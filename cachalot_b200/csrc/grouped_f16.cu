@@ -535,10 +535,9 @@ F16Scratch carve_f16(uint8_t* base, const BankView& v, size_t R, size_t n_seg) {
   s.plan.units = reinterpret_cast<Unit*>(take((R / NT + R + 1) * sizeof(Unit)));  // a segment with rows: ceil(rows / NT)
   s.x_scale = reinterpret_cast<float*>(take(R * 4));
   s.h_scale = reinterpret_cast<float*>(take(R * 4));
-  s.xp = reinterpret_cast<__half*>(take(R * k_shape(v.hidden, v.group).pitch * 2));
-  s.h = reinterpret_cast<__nv_bfloat16*>(take(R * v.inter * 2));
-  s.hp = reinterpret_cast<__half*>(take(R * k_shape(v.inter, v.group).pitch * 2));
-  s.y = reinterpret_cast<__nv_bfloat16*>(take(R * v.hidden * 2));
+  // x is through when h is prepared, and h when y is written: two buffers serve the four
+  s.xp = s.hp = reinterpret_cast<__half*>(take(R * max(k_shape(v.hidden, v.group).pitch, k_shape(v.inter, v.group).pitch) * 2));
+  s.h = s.y = reinterpret_cast<__nv_bfloat16*>(take(R * max(v.hidden, v.inter) * 2));
   s.total = at;
   return s;
 }

@@ -282,7 +282,7 @@ PyObject* prefill_grouped(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   PLAIN_OR_NONE(t > 0 && k > 0 && t * k < (1 << 30) && x->size(0) == t && w->size(0) == t && w->size(1) == k);
   const size_t perm = up256((size_t)t * k * 4), offs = up256((size_t)(e + 1) * 4);
   const size_t counts = up256(cachalot_group_rows_scratch_ints((int)t, (int)k, (int)e) * 4);
-  const size_t need = cachalot_moe_prefill_workspace_bytes(d, (int)t, (int)k, mx);
+  const size_t need = cachalot_moe_prefill_experts_workspace_bytes(d, (int)t, (int)k, (int)e, mx);
   const at::Tensor ws = scratch(perm + offs + counts + need, dev);
   at::Tensor out = empty({t, d->hidden}, ScalarType::Float, dev);
   uint8_t* b = static_cast<uint8_t*>(ws.data_ptr());

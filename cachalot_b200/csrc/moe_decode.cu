@@ -505,12 +505,25 @@ static size_t prefill_min_workspace(const cachalot_bank_desc* desc, int tokens, 
   return b;
 }
 
+static bool prefill_f16_takes(const BankView& v, int tokens, int k, int n_experts, int mxfp4_act) {
+  return !mxfp4_act && f16_supported(v) && n_experts <= 8192 && grouped_f16_pays(v, tokens, k, n_experts);
+}
+
 extern "C" size_t cachalot_moe_prefill_workspace_bytes(const cachalot_bank_desc* desc, int tokens, int k, int mxfp4_act) {
   if (!desc || tokens <= 0 || k <= 0) return 0;
   const size_t b = prefill_min_workspace(desc, tokens, k, mxfp4_act);
   const BankView v = shape_view(desc);
-  if (mxfp4_act || !f16_supported(v) || (long long)tokens * k > 65535) return b;
-  const size_t f = prefill_f16_workspace_bytes(v, tokens, k, 8192);  // the expert count is not known here
+  if (!prefill_f16_takes(v, tokens, k, 1, mxfp4_act) || (long long)tokens * k > 65535) return b;
+  const size_t f = prefill_f16_workspace_bytes(v, tokens, k, 8192);  // enough for any number of experts
+  return f > b ? f : b;
+}
+
+extern "C" size_t cachalot_moe_prefill_experts_workspace_bytes(const cachalot_bank_desc* desc, int tokens, int k, int n_experts, int mxfp4_act) {
+  if (!desc || tokens <= 0 || k <= 0 || n_experts <= 0) return 0;
+  const size_t b = prefill_min_workspace(desc, tokens, k, mxfp4_act);
+  const BankView v = shape_view(desc);
+  if (!prefill_f16_takes(v, tokens, k, n_experts, mxfp4_act) || (long long)tokens * k > 65535) return b;
+  const size_t f = prefill_f16_workspace_bytes(v, tokens, k, n_experts);
   return f > b ? f : b;
 }
 
@@ -540,7 +553,7 @@ extern "C" int cachalot_moe_prefill(const void* bank, const cachalot_bank_desc* 
   if (tc)
     return launch_prefill_tc(v, x_bf16, perm, offsets, slot_of_expert, gate_w, tokens, k, n_experts, swiglu_limit, workspace, out,
                              status, s);
-  if (!mxfp4_act && f16_supported(v) && n_experts <= 8192 && grouped_f16_pays(v, tokens, k, n_experts) &&
+  if (prefill_f16_takes(v, tokens, k, n_experts, mxfp4_act) &&
       workspace_bytes >= prefill_f16_workspace_bytes(v, tokens, k, n_experts))
     return launch_prefill_f16(v, x_bf16, perm, offsets, slot_of_expert, gate_w, tokens, k, n_experts, swiglu_limit, workspace, out, status, s);
   uint8_t* ws = static_cast<uint8_t*>(workspace);

@@ -532,7 +532,7 @@ def moe_prefill_grouped(x: torch.Tensor, expert_ids: torch.Tensor, weights: torc
     out = torch.empty((t, bank.hidden), dtype=torch.float32, device=x.device)
     if t == 0:
         return out
-    need = lib.cachalot_moe_prefill_workspace_bytes(bank.desc_ptr, t, k, int(mxfp4_act))
+    need = lib.cachalot_moe_prefill_experts_workspace_bytes(bank.desc_ptr, t, k, e, int(mxfp4_act))
     ws = _workspace(x.device, need + 256)
     base = (ws.data_ptr() + 255) // 256 * 256
     check(lib.cachalot_moe_prefill(_ptr(bank.slab), bank.desc_ptr, _ptr(xb), _ptr(perm), _ptr(offsets), _ptr(slot_of_expert),

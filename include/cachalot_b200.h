@@ -185,7 +185,7 @@ CACHALOT_API int cachalot_moe_layer_decode(const void* bank, const cachalot_bank
  * synchronisation in the middle of a token), a plugin slot whose signature has no room for a
  * scratch pointer, or a real-time decode loop that may not call into the allocator.  The scratch is
  * a 4 MiB array that is part of the library image: every GPU that loads the library holds it until
- * the process exits.  A call whose cachalot_moe_decode_workspace_bytes(desc, rows, k) exceeds
+ * the process exits.  A call that cannot do with
  * cachalot_moe_decode_static_scratch_bytes() is refused with CACHALOT_ESCRATCH and nothing is
  * launched (decode batches of a few tokens fit; larger ones need the caller's own workspace).  The
  * entry point calls no cudaMalloc, cudaFree or other allocating routine.
@@ -266,8 +266,14 @@ CACHALOT_API int cachalot_group_rows(const int32_t* expert_ids, int tokens, int 
 CACHALOT_API int cachalot_mxfp4_act_quant(const void* x_bf16, const int32_t* src_rows, int rows, int k, uint8_t* codes,
                              uint8_t* scales, cachalot_stream_t stream);
 
+/* Scratch of cachalot_moe_prefill: enough for any number of experts, or for n_experts of them (less where the call does
+ * not take the grouped kernels of a 2-bit bank).  A 2-bit bank runs with less than this, down to
+ * tokens * k * (4 * inter + 4) bytes and two roundings to 256, but then token by token: about a tenth of the speed for
+ * chunks of many tokens. */
 CACHALOT_API size_t cachalot_moe_prefill_workspace_bytes(const cachalot_bank_desc* desc /* host */, int tokens, int k,
                                             int mxfp4_act);
+CACHALOT_API size_t cachalot_moe_prefill_experts_workspace_bytes(const cachalot_bank_desc* desc /* host */, int tokens, int k,
+                                                    int n_experts, int mxfp4_act);
 
 /* Replaces the expert loop and combine of model/moe_prefill_grouped.py:384-530 with
  * model/fp4_sgmm_metal.py:318-333 / model/moe_prefill_batched.py:31-61 /

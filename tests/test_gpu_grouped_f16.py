@@ -84,6 +84,32 @@ def test_stages_with_one_operand_slot(hidden, inter, group):
     assert within_bf16_flips(got[some].cpu().numpy(), _want(x[some], slots[some], w[some], experts, group))
 
 
+@pytest.mark.parametrize("general", [False, True])
+@pytest.mark.parametrize("tokens,experts,grouped", [(64, 128, False), (512, 128, True)])
+def test_prefill_scratch(tokens, experts, grouped, general):
+    """A chunk that goes token by token takes the scratch of that route only; a grouped one two buffers of 16-bit rows."""
+    import torch
+
+    import cachalot_b200 as cb
+
+    hidden, inter, k = 4096, 2880, 6
+    bank = cb.SlabBank(cb.affine_format(hidden, inter), hidden, inter, experts, layers=1, n_experts=experts)
+    bank.fill_random(torch.Generator(device="cuda").manual_seed(1))
+    x = torch.randn((tokens, hidden), device="cuda").to(torch.bfloat16)
+    ids = torch.rand((tokens, experts), device="cuda").topk(k, 1).indices.to(torch.int32)
+    w = torch.rand((tokens, k), device="cuda")
+    args = (x.float() if general else x, ids, w, bank)
+    cb.ops._workspaces.clear()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    out = cb.moe_prefill_grouped(*args)
+    used = torch.cuda.max_memory_allocated() - before - out.numel() * 4 - (x.numel() * 2 if general else 0)
+    rows = tokens * k
+    need = rows * 2 * (hidden + 128 + hidden) if grouped else rows * inter * 4
+    assert used <= need + rows * 64 + (2 << 20), f"{used} bytes for {rows} rows"
+
+
 def test_infinite_and_nan_activations():
     """An infinite or NaN activation does to its row, and to no other, what it does in the one-token kernel.  All biases of
     these banks are negative: -inf drives gate and up to +inf, which the clamp makes finite again, as it does NaN; +inf ends
