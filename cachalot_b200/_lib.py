@@ -94,8 +94,7 @@ def _load() -> C.CDLL:
             f"{LIB_PATH} is missing: build it with `python -m cachalot_b200.build` "
             "(needs nvcc; there is no CPU or PyTorch fallback for these kernels)"
         )
-    # an override goes into the global scope, where the native call path (_host.so) finds it before its own copy
-    lib = C.CDLL(str(LIB_PATH), mode=C.RTLD_GLOBAL if "CACHALOT_B200_LIB" in os.environ else C.DEFAULT_MODE)
+    lib = C.CDLL(str(LIB_PATH))
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError if the symbol is not exported
         fn.restype, fn.argtypes = res, args
@@ -103,6 +102,19 @@ def _load() -> C.CDLL:
 
 
 lib = _load()
+
+
+def load_host():
+    """The native call path of the operators (csrc/host/host.cpp), bound to the entry points of `lib`."""
+    rebuild = "build it with `python -m cachalot_b200.build` (it is compiled against the installed Python and torch)"
+    if not (_PKG / "_host.so").exists():
+        raise ImportError(f"{_PKG / '_host.so'} is missing: {rebuild}")
+    try:
+        from . import _host
+    except ImportError as e:
+        raise ImportError(f"{_PKG / '_host.so'} does not load ({e}): {rebuild}") from e
+    _host.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in _host.entries()})
+    return _host
 
 
 def last_error() -> str:

@@ -3,7 +3,8 @@
 `python -m cachalot_b200.build` (or `build()` from Python) compiles every `csrc/*.cu` with
 nvcc into `cachalot_b200/libcachalot_b200.so` (nvcc cross-compiles without a GPU) and
 `csrc/host/host.cpp` with the C++ compiler into the extension module `cachalot_b200/_host.so`.
-Each is rebuilt only when a source or header is newer than it.
+Each is rebuilt only when a source or header is newer than it.  CACHALOT_B200_LIB names another file for the library
+(development builds); the extension module is the same for all of them.
 """
 from __future__ import annotations
 
@@ -13,6 +14,7 @@ import subprocess
 import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
+from importlib import metadata
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -21,6 +23,7 @@ LIB = Path(os.environ.get("CACHALOT_B200_LIB", PKG / "libcachalot_b200.so"))
 OBJ_DIR = PKG / "csrc" / "build"
 HOST_SRC = CSRC / "host" / "host.cpp"
 HOST_LIB = PKG / "_host.so"
+HOST_STAMP = OBJ_DIR / "host.stamp"  # what _host.so was compiled for
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -53,9 +56,12 @@ def needs_build() -> bool:
 
 
 def build_host(force: bool = False) -> Path:
-    """The extension module that ops.py calls (it links the CUDA library beside it by its own location)."""
+    """The extension module that ops.py calls.  It takes the CUDA library's entry points as addresses (_lib.load_host)
+    and links torch only; it is built anew for another Python or torch."""
     deps = [HOST_SRC, PKG.parent / "include" / "cachalot_b200.h"]
-    if not force and HOST_LIB.exists() and all(p.stat().st_mtime <= HOST_LIB.stat().st_mtime for p in deps):
+    made_for = f"python {sys.version}\ntorch {metadata.version('torch')}\n"
+    if not force and HOST_LIB.exists() and HOST_STAMP.exists() and HOST_STAMP.read_text() == made_for and \
+            all(p.stat().st_mtime <= HOST_LIB.stat().st_mtime for p in deps):
         return HOST_LIB
     from torch.utils import cpp_extension
 
@@ -63,10 +69,12 @@ def build_host(force: bool = False) -> Path:
            f"-D_GLIBCXX_USE_CXX11_ABI={int(_torch_cxx11_abi())}", "-I" + sysconfig.get_paths()["include"],
            "-I" + str(Path(_nvcc()).resolve().parents[1] / "include"), *("-isystem" + p for p in cpp_extension.include_paths()),
            str(HOST_SRC), "-o", str(HOST_LIB), *("-L" + p for p in cpp_extension.library_paths()), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
-           "-lc10_cuda", "-lc10", "-L" + str(LIB.parent), "-l:" + LIB.name, "-Wl,-rpath,$ORIGIN"]
+           "-lc10_cuda", "-lc10"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"host module failed:\n{res.stdout}\n{res.stderr}")
+    OBJ_DIR.mkdir(exist_ok=True)
+    HOST_STAMP.write_text(made_for)
     return HOST_LIB
 
 

@@ -24,6 +24,48 @@ namespace {
 
 using at::ScalarType;
 
+// The entry points of the C ABI, as the addresses _lib.py found in the library it loaded (by default the one beside this
+// module, else CACHALOT_B200_LIB): this module links no library of its own, so both ways of a call end in the same one.
+#define ENTRIES(X) \
+  X(cachalot_bf16_gemv_f32) X(cachalot_fp8_linear) X(cachalot_group_rows) X(cachalot_group_rows_scratch_ints) \
+  X(cachalot_last_error) X(cachalot_moe_decode) X(cachalot_moe_decode_workspace_bytes) X(cachalot_moe_layer_decode) \
+  X(cachalot_moe_layer_decode_workspace_bytes) X(cachalot_moe_prefill) X(cachalot_moe_prefill_experts_workspace_bytes) X(cachalot_route_topk) \
+  X(cachalot_router_logits) X(cachalot_shared_expert) X(cachalot_shared_expert_workspace_bytes)
+struct Lib {
+#define X(name) decltype(&::name) name = nullptr;
+  ENTRIES(X)
+#undef X
+} lib;
+bool bound = false;
+
+// () -> names of the entry points
+PyObject* entries(PyObject*, PyObject* const*, Py_ssize_t) {
+#define X(name) #name,
+  const char* const all[] = {ENTRIES(X)};
+#undef X
+  PyObject* out = PyList_New(0);
+  for (const char* n : all) {
+    PyObject* s = out ? PyUnicode_FromString(n) : nullptr;
+    if (!s || PyList_Append(out, s) < 0) Py_CLEAR(out);
+    Py_XDECREF(s);
+  }
+  return out;
+}
+// ({name: address}) -> None
+PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  if (n_args != 1 || !PyDict_Check(a[0])) return PyErr_Format(PyExc_TypeError, "bind takes a dict of addresses");
+  Lib l;
+  void* p;
+#define X(name)                                                                                              \
+  p = PyDict_GetItemString(a[0], #name) ? PyLong_AsVoidPtr(PyDict_GetItemString(a[0], #name)) : nullptr;     \
+  if (!p) return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_ValueError, "no address for " #name);       \
+  l.name = reinterpret_cast<decltype(l.name)>(p);
+  ENTRIES(X)
+#undef X
+  lib = l, bound = true;
+  Py_RETURN_NONE;
+}
+
 const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 
 // a contiguous tensor of this type on the current device?
@@ -52,7 +94,7 @@ cachalot_stream_t current_stream(int device) {
 // the exception a return code of the C ABI stands for (as _lib.check)
 PyObject* raise(int rc) {
   PyObject* type = rc == CACHALOT_EUNSUPPORTED ? PyExc_NotImplementedError : rc == CACHALOT_ECUDA ? PyExc_RuntimeError : PyExc_ValueError;
-  PyErr_SetString(type, cachalot_last_error());
+  PyErr_SetString(type, lib.cachalot_last_error());
   return nullptr;
 }
 
@@ -102,7 +144,7 @@ int fp8_block(const at::Tensor* s, int64_t n, int64_t k, int device, int* rule) 
 // (x, weight, weight_scales, out dtype) -> y
 PyObject* fp8_linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  PLAIN_OR_NONE(n_args == 4);
+  PLAIN_OR_NONE(bound && n_args == 4);
   Args p{a};
   const int dev = current_device(), odt = (int)p.i(3);
   const at::Tensor *x = tensor_of(a[0]), *w = tensor_of(a[1]), *s = tensor_of(a[2]);
@@ -116,7 +158,7 @@ PyObject* fp8_linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const at::Tensor ws = scratch(codes_bytes + (size_t)rows * (k / block) * 4, dev);
   at::Tensor y = x->dim() == 1 ? empty({n}, out_type(odt), dev) : empty({rows, n}, out_type(odt), dev);
   uint8_t* codes = static_cast<uint8_t*>(ws.data_ptr());
-  const int rc = cachalot_fp8_linear(x->data_ptr(), (int)rows, (int)k, block, rule, codes, reinterpret_cast<float*>(codes + codes_bytes),
+  const int rc = lib.cachalot_fp8_linear(x->data_ptr(), (int)rows, (int)k, block, rule, codes, reinterpret_cast<float*>(codes + codes_bytes),
                                      static_cast<const uint8_t*>(w->data_ptr()), s->data_ptr(), (int)n, y.data_ptr(), odt, current_stream(dev));
   if (rc) return raise(rc);
   return THPVariable_Wrap(std::move(y));
@@ -126,7 +168,7 @@ PyObject* fp8_linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 // (x f32, weight bf16) -> y f32
 PyObject* bf16_gemv_f32(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  PLAIN_OR_NONE(n_args == 2);
+  PLAIN_OR_NONE(bound && n_args == 2);
   const int dev = current_device();
   const at::Tensor *x = tensor_of(a[0]), *w = tensor_of(a[1]);
   PLAIN_OR_NONE(plain(x, ScalarType::Float, dev) && plain(w, ScalarType::BFloat16, dev) && w->dim() == 2 && (x->dim() == 1 || x->dim() == 2));
@@ -135,7 +177,7 @@ PyObject* bf16_gemv_f32(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   at::Tensor y = x->dim() == 1 ? empty({n}, ScalarType::Float, dev) : empty({rows, n}, ScalarType::Float, dev);
   const cachalot_stream_t st = current_stream(dev);
   for (int64_t r = 0; r < rows; r += 8) {
-    const int rc = cachalot_bf16_gemv_f32(static_cast<const float*>(x->data_ptr()) + r * k, (int)(rows - r < 8 ? rows - r : 8), w->data_ptr(),
+    const int rc = lib.cachalot_bf16_gemv_f32(static_cast<const float*>(x->data_ptr()) + r * k, (int)(rows - r < 8 ? rows - r : 8), w->data_ptr(),
                                           (int)n, (int)k, static_cast<float*>(y.data_ptr()) + r * n, st);
     if (rc) return raise(rc);
   }
@@ -163,9 +205,9 @@ bool shared_from(PyObject* const* a, int64_t hidden, int dev, Shared* m) {  // w
   return m->w3->size(0) == m->inter && m->w3->size(1) == hidden && fp8_block(m->s3, m->inter, hidden, dev, &r3) == m->block && r3 == m->rule;
 }
 int run_shared(const void* x, int64_t rows, const Shared& m, double limit, const float* addend, void* out, int dev) {
-  const size_t need = cachalot_shared_expert_workspace_bytes((int)rows, (int)m.hidden, (int)m.inter, m.block);
+  const size_t need = lib.cachalot_shared_expert_workspace_bytes((int)rows, (int)m.hidden, (int)m.inter, m.block);
   const at::Tensor ws = scratch(need, dev);
-  return cachalot_shared_expert(x, (int)rows, (int)m.hidden, (int)m.inter, static_cast<const uint8_t*>(m.w1->data_ptr()), m.s1->data_ptr(),
+  return lib.cachalot_shared_expert(x, (int)rows, (int)m.hidden, (int)m.inter, static_cast<const uint8_t*>(m.w1->data_ptr()), m.s1->data_ptr(),
                                 m.w3 ? static_cast<const uint8_t*>(m.w3->data_ptr()) : nullptr, m.w3 ? m.s3->data_ptr() : nullptr,
                                 static_cast<const uint8_t*>(m.w2->data_ptr()), m.s2->data_ptr(), m.rule, m.block, (float)limit, addend,
                                 ws.data_ptr(), (size_t)ws.numel(), out, current_stream(dev));
@@ -174,7 +216,7 @@ int run_shared(const void* x, int64_t rows, const Shared& m, double limit, const
 // (x, w1, s1, w3 | None, s3 | None, w2, s2, limit) -> y bf16, in x's shape
 PyObject* shared_expert(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  PLAIN_OR_NONE(n_args == 8);
+  PLAIN_OR_NONE(bound && n_args == 8);
   Args p{a};
   const int dev = current_device();
   const at::Tensor* x = tensor_of(a[0]);
@@ -193,7 +235,7 @@ PyObject* shared_expert(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 // (x [rows, H], slots [rows, k], gate weights [rows, k], slab, descriptor, limit, numerics, out dtype, status | None) -> out [rows, H]
 PyObject* moe_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  PLAIN_OR_NONE(n_args == 9);
+  PLAIN_OR_NONE(bound && n_args == 9);
   Args p{a};
   const int dev = current_device(), num = (int)p.i(6), odt = (int)p.i(7);
   const double limit = p.f(5);
@@ -205,8 +247,8 @@ PyObject* moe_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const int64_t rows = x->size(0), k = slots->size(1);
   PLAIN_OR_NONE(rows > 0 && rows < (1 << 30) && slots->size(0) == rows && gw->size(0) == rows && gw->size(1) == k && k > 0 && k < 1024);
   at::Tensor out = empty({rows, d->hidden}, out_type(odt), dev);
-  const at::Tensor ws = scratch(cachalot_moe_decode_workspace_bytes(d, (int)rows, (int)k), dev);
-  const int rc = cachalot_moe_decode(slab->data_ptr(), d, x->data_ptr(), static_cast<const int32_t*>(slots->data_ptr()),
+  const at::Tensor ws = scratch(lib.cachalot_moe_decode_workspace_bytes(d, (int)rows, (int)k), dev);
+  const int rc = lib.cachalot_moe_decode(slab->data_ptr(), d, x->data_ptr(), static_cast<const int32_t*>(slots->data_ptr()),
                                      static_cast<const float*>(gw->data_ptr()), (int)rows, (int)k, (float)limit, num, ws.data_ptr(),
                                      (size_t)ws.numel(), out.data_ptr(), odt, static_cast<int*>(ptr_or_null(a[8])), current_stream(dev));
   if (rc) return raise(rc);
@@ -223,8 +265,8 @@ struct LayerCall {  // what a one-token layer takes besides x and the logits
   int* status;
 };
 int run_layer(const LayerCall& c, const void* x, const float* logits, void* out, int32_t* idx, float* w, int dev) {
-  const at::Tensor ws = scratch(cachalot_moe_layer_decode_workspace_bytes(c.d, c.topk), dev);
-  return cachalot_moe_layer_decode(c.slab->data_ptr(), c.d, x, logits, c.bias, static_cast<const int32_t*>(c.table->data_ptr()), c.layer,
+  const at::Tensor ws = scratch(lib.cachalot_moe_layer_decode_workspace_bytes(c.d, c.topk), dev);
+  return lib.cachalot_moe_layer_decode(c.slab->data_ptr(), c.d, x, logits, c.bias, static_cast<const int32_t*>(c.table->data_ptr()), c.layer,
                                    c.experts, c.topk, c.mode, (float)c.temp, (float)c.scale, c.norm, c.weights_bf16, (float)c.limit, c.numerics,
                                    ws.data_ptr(), (size_t)ws.numel(), out, c.odt, idx, w, c.status, current_stream(dev));
 }
@@ -236,7 +278,7 @@ bool table_fits(const at::Tensor* t, int layer, int64_t experts, int dev) {
 //  out dtype, out | None, status | None, want_routing) -> out, or (out, indices, weights)
 PyObject* layer_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  PLAIN_OR_NONE(n_args == 19);
+  PLAIN_OR_NONE(bound && n_args == 19);
   Args p{a};
   const int dev = current_device();
   const at::Tensor *x = tensor_of(a[0]), *logits = tensor_of(a[1]);
@@ -268,7 +310,7 @@ PyObject* layer_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 // (x [T, H], expert_ids [T, k], weights [T, k], slab, descriptor, table, layer, experts, limit, mxfp4_act, status | None) -> out f32 [T, H]
 PyObject* prefill_grouped(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  PLAIN_OR_NONE(n_args == 11);
+  PLAIN_OR_NONE(bound && n_args == 11);
   Args p{a};
   const int dev = current_device(), layer = (int)p.i(6), mx = (int)p.i(9);
   const int64_t e = p.i(7);
@@ -281,17 +323,17 @@ PyObject* prefill_grouped(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const int64_t t = ids->size(0), k = ids->size(1);
   PLAIN_OR_NONE(t > 0 && k > 0 && t * k < (1 << 30) && x->size(0) == t && w->size(0) == t && w->size(1) == k);
   const size_t perm = up256((size_t)t * k * 4), offs = up256((size_t)(e + 1) * 4);
-  const size_t counts = up256(cachalot_group_rows_scratch_ints((int)t, (int)k, (int)e) * 4);
-  const size_t need = cachalot_moe_prefill_experts_workspace_bytes(d, (int)t, (int)k, (int)e, mx);
+  const size_t counts = up256(lib.cachalot_group_rows_scratch_ints((int)t, (int)k, (int)e) * 4);
+  const size_t need = lib.cachalot_moe_prefill_experts_workspace_bytes(d, (int)t, (int)k, (int)e, mx);
   const at::Tensor ws = scratch(perm + offs + counts + need, dev);
   at::Tensor out = empty({t, d->hidden}, ScalarType::Float, dev);
   uint8_t* b = static_cast<uint8_t*>(ws.data_ptr());
   int32_t *pm = reinterpret_cast<int32_t*>(b), *of = reinterpret_cast<int32_t*>(b + perm), *ct = reinterpret_cast<int32_t*>(b + perm + offs);
   int* status = static_cast<int*>(ptr_or_null(a[10]));
   const cachalot_stream_t st = current_stream(dev);
-  int rc = cachalot_group_rows(static_cast<const int32_t*>(ids->data_ptr()), (int)t, (int)k, (int)e, pm, of, ct, status, st);
+  int rc = lib.cachalot_group_rows(static_cast<const int32_t*>(ids->data_ptr()), (int)t, (int)k, (int)e, pm, of, ct, status, st);
   if (!rc)
-    rc = cachalot_moe_prefill(slab->data_ptr(), d, x->data_ptr(), pm, of, static_cast<const int32_t*>(table->data_ptr()) + (size_t)layer * e,
+    rc = lib.cachalot_moe_prefill(slab->data_ptr(), d, x->data_ptr(), pm, of, static_cast<const int32_t*>(table->data_ptr()) + (size_t)layer * e,
                               static_cast<const float*>(w->data_ptr()), (int)t, (int)k, (int)e, (float)limit, mx, b + perm + offs + counts,
                               (size_t)ws.numel() - perm - offs - counts, static_cast<float*>(out.data_ptr()), status, st);
   if (rc) return raise(rc);
@@ -303,7 +345,7 @@ PyObject* prefill_grouped(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 //  w1, s1, w3 | None, s3 | None, w2, s2) -> (out bf16 [H], indices, weights, scores | None)
 PyObject* moe_block(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  PLAIN_OR_NONE(n_args == 21);
+  PLAIN_OR_NONE(bound && n_args == 21);
   Args p{a};
   const int dev = current_device();
   const at::Tensor *x = tensor_of(a[0]), *gate = tensor_of(a[1]), *bias = tensor_of(a[2]);
@@ -331,9 +373,9 @@ PyObject* moe_block(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   int32_t* ip = static_cast<int32_t*>(idx.data_ptr());
   float* wp = static_cast<float*>(w.data_ptr());
   const cachalot_stream_t st = current_stream(dev);
-  int rc = cachalot_router_logits(x->data_ptr(), gate->data_ptr(), gate_bf16 ? CACHALOT_BF16 : CACHALOT_F32, 1, (int)e, (int)h, logits, st);
+  int rc = lib.cachalot_router_logits(x->data_ptr(), gate->data_ptr(), gate_bf16 ? CACHALOT_BF16 : CACHALOT_F32, 1, (int)e, (int)h, logits, st);
   if (!rc && want_scores)
-    rc = cachalot_route_topk(logits, c.bias, nullptr, 0, 1, (int)e, c.topk, c.mode, (float)c.temp, (float)c.scale, c.norm, 0, ip, wp, nullptr,
+    rc = lib.cachalot_route_topk(logits, c.bias, nullptr, 0, 1, (int)e, c.topk, c.mode, (float)c.temp, (float)c.scale, c.norm, 0, ip, wp, nullptr,
                              static_cast<float*>(sc.data_ptr()), st);
   if (!rc) rc = run_layer(c, x->data_ptr(), logits, routed, ip, wp, dev);
   if (!rc) rc = run_shared(x->data_ptr(), 1, m, c.limit, routed, out.data_ptr(), dev);
@@ -344,7 +386,7 @@ PyObject* moe_block(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 }
 
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(fp8_linear), FAST(bf16_gemv_f32), FAST(shared_expert), FAST(moe_forward), FAST(layer_decode),
+PyMethodDef methods[] = {FAST(entries), FAST(bind), FAST(fp8_linear), FAST(bf16_gemv_f32), FAST(shared_expert), FAST(moe_forward), FAST(layer_decode),
                          FAST(prefill_grouped), FAST(moe_block), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native call path of the operators (see host.cpp).", -1, methods};
 

@@ -12,11 +12,12 @@ from dataclasses import dataclass
 
 import torch
 
-from . import _host, _lib
+from . import _lib
 from ._lib import check, lib
 from .bank import FP4_FORMAT, ExpertFormat, ResidentExpert, SlabBank
 
 
+_host = _lib.load_host()
 _ODT = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16}
 _NUMERICS = {"f32": _lib.NUMERICS_F32, "bf16": _lib.NUMERICS_BF16, "bf16_h32": _lib.NUMERICS_BF16_H32}
 _ROUTER = {"sigmoid": _lib.ROUTER_SIGMOID, "sqrt_softplus": _lib.ROUTER_SQRT_SOFTPLUS}
