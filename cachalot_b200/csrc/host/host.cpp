@@ -98,6 +98,18 @@ PyObject* raise(int rc) {
   return nullptr;
 }
 
+// Launches without the interpreter's lock, as ctypes makes them: a call that fills the launch queue (a launch per token, or
+// calls far ahead of the GPU) waits in the driver, and other Python threads run meanwhile.
+template <typename F>
+int unlocked(F&& launch) {
+  struct Unlock {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Unlock() { PyEval_RestoreThread(state); }
+  } u;
+  return launch();
+}
+#define UNLOCKED(call) unlocked([&] { return call; })
+
 // numeric arguments
 struct Args {
   PyObject* const* a;
@@ -158,8 +170,9 @@ PyObject* fp8_linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const at::Tensor ws = scratch(codes_bytes + (size_t)rows * (k / block) * 4, dev);
   at::Tensor y = x->dim() == 1 ? empty({n}, out_type(odt), dev) : empty({rows, n}, out_type(odt), dev);
   uint8_t* codes = static_cast<uint8_t*>(ws.data_ptr());
-  const int rc = lib.cachalot_fp8_linear(x->data_ptr(), (int)rows, (int)k, block, rule, codes, reinterpret_cast<float*>(codes + codes_bytes),
-                                     static_cast<const uint8_t*>(w->data_ptr()), s->data_ptr(), (int)n, y.data_ptr(), odt, current_stream(dev));
+  const int rc = UNLOCKED(lib.cachalot_fp8_linear(x->data_ptr(), (int)rows, (int)k, block, rule, codes,
+                                                  reinterpret_cast<float*>(codes + codes_bytes), static_cast<const uint8_t*>(w->data_ptr()),
+                                                  s->data_ptr(), (int)n, y.data_ptr(), odt, current_stream(dev)));
   if (rc) return raise(rc);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
@@ -177,8 +190,8 @@ PyObject* bf16_gemv_f32(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   at::Tensor y = x->dim() == 1 ? empty({n}, ScalarType::Float, dev) : empty({rows, n}, ScalarType::Float, dev);
   const cachalot_stream_t st = current_stream(dev);
   for (int64_t r = 0; r < rows; r += 8) {
-    const int rc = lib.cachalot_bf16_gemv_f32(static_cast<const float*>(x->data_ptr()) + r * k, (int)(rows - r < 8 ? rows - r : 8), w->data_ptr(),
-                                          (int)n, (int)k, static_cast<float*>(y.data_ptr()) + r * n, st);
+    const int rc = UNLOCKED(lib.cachalot_bf16_gemv_f32(static_cast<const float*>(x->data_ptr()) + r * k, (int)(rows - r < 8 ? rows - r : 8),
+                                                       w->data_ptr(), (int)n, (int)k, static_cast<float*>(y.data_ptr()) + r * n, st));
     if (rc) return raise(rc);
   }
   return THPVariable_Wrap(std::move(y));
@@ -207,10 +220,10 @@ bool shared_from(PyObject* const* a, int64_t hidden, int dev, Shared* m) {  // w
 int run_shared(const void* x, int64_t rows, const Shared& m, double limit, const float* addend, void* out, int dev) {
   const size_t need = lib.cachalot_shared_expert_workspace_bytes((int)rows, (int)m.hidden, (int)m.inter, m.block);
   const at::Tensor ws = scratch(need, dev);
-  return lib.cachalot_shared_expert(x, (int)rows, (int)m.hidden, (int)m.inter, static_cast<const uint8_t*>(m.w1->data_ptr()), m.s1->data_ptr(),
+  return UNLOCKED(lib.cachalot_shared_expert(x, (int)rows, (int)m.hidden, (int)m.inter, static_cast<const uint8_t*>(m.w1->data_ptr()), m.s1->data_ptr(),
                                 m.w3 ? static_cast<const uint8_t*>(m.w3->data_ptr()) : nullptr, m.w3 ? m.s3->data_ptr() : nullptr,
                                 static_cast<const uint8_t*>(m.w2->data_ptr()), m.s2->data_ptr(), m.rule, m.block, (float)limit, addend,
-                                ws.data_ptr(), (size_t)ws.numel(), out, current_stream(dev));
+                                ws.data_ptr(), (size_t)ws.numel(), out, current_stream(dev)));
 }
 
 // (x, w1, s1, w3 | None, s3 | None, w2, s2, limit) -> y bf16, in x's shape
@@ -248,9 +261,10 @@ PyObject* moe_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   PLAIN_OR_NONE(rows > 0 && rows < (1 << 30) && slots->size(0) == rows && gw->size(0) == rows && gw->size(1) == k && k > 0 && k < 1024);
   at::Tensor out = empty({rows, d->hidden}, out_type(odt), dev);
   const at::Tensor ws = scratch(lib.cachalot_moe_decode_workspace_bytes(d, (int)rows, (int)k), dev);
-  const int rc = lib.cachalot_moe_decode(slab->data_ptr(), d, x->data_ptr(), static_cast<const int32_t*>(slots->data_ptr()),
+  int* status = static_cast<int*>(ptr_or_null(a[8]));
+  const int rc = UNLOCKED(lib.cachalot_moe_decode(slab->data_ptr(), d, x->data_ptr(), static_cast<const int32_t*>(slots->data_ptr()),
                                      static_cast<const float*>(gw->data_ptr()), (int)rows, (int)k, (float)limit, num, ws.data_ptr(),
-                                     (size_t)ws.numel(), out.data_ptr(), odt, static_cast<int*>(ptr_or_null(a[8])), current_stream(dev));
+                                     (size_t)ws.numel(), out.data_ptr(), odt, status, current_stream(dev)));
   if (rc) return raise(rc);
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -266,9 +280,9 @@ struct LayerCall {  // what a one-token layer takes besides x and the logits
 };
 int run_layer(const LayerCall& c, const void* x, const float* logits, void* out, int32_t* idx, float* w, int dev) {
   const at::Tensor ws = scratch(lib.cachalot_moe_layer_decode_workspace_bytes(c.d, c.topk), dev);
-  return lib.cachalot_moe_layer_decode(c.slab->data_ptr(), c.d, x, logits, c.bias, static_cast<const int32_t*>(c.table->data_ptr()), c.layer,
+  return UNLOCKED(lib.cachalot_moe_layer_decode(c.slab->data_ptr(), c.d, x, logits, c.bias, static_cast<const int32_t*>(c.table->data_ptr()), c.layer,
                                    c.experts, c.topk, c.mode, (float)c.temp, (float)c.scale, c.norm, c.weights_bf16, (float)c.limit, c.numerics,
-                                   ws.data_ptr(), (size_t)ws.numel(), out, c.odt, idx, w, c.status, current_stream(dev));
+                                   ws.data_ptr(), (size_t)ws.numel(), out, c.odt, idx, w, c.status, current_stream(dev)));
 }
 bool table_fits(const at::Tensor* t, int layer, int64_t experts, int dev) {
   return plain(t, ScalarType::Int, dev) && t->dim() == 2 && t->size(1) == experts && layer >= 0 && layer < t->size(0);
@@ -331,11 +345,12 @@ PyObject* prefill_grouped(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   int32_t *pm = reinterpret_cast<int32_t*>(b), *of = reinterpret_cast<int32_t*>(b + perm), *ct = reinterpret_cast<int32_t*>(b + perm + offs);
   int* status = static_cast<int*>(ptr_or_null(a[10]));
   const cachalot_stream_t st = current_stream(dev);
-  int rc = lib.cachalot_group_rows(static_cast<const int32_t*>(ids->data_ptr()), (int)t, (int)k, (int)e, pm, of, ct, status, st);
+  int rc = UNLOCKED(lib.cachalot_group_rows(static_cast<const int32_t*>(ids->data_ptr()), (int)t, (int)k, (int)e, pm, of, ct, status, st));
   if (!rc)
-    rc = lib.cachalot_moe_prefill(slab->data_ptr(), d, x->data_ptr(), pm, of, static_cast<const int32_t*>(table->data_ptr()) + (size_t)layer * e,
+    rc = UNLOCKED(lib.cachalot_moe_prefill(slab->data_ptr(), d, x->data_ptr(), pm, of,
+                              static_cast<const int32_t*>(table->data_ptr()) + (size_t)layer * e,
                               static_cast<const float*>(w->data_ptr()), (int)t, (int)k, (int)e, (float)limit, mx, b + perm + offs + counts,
-                              (size_t)ws.numel() - perm - offs - counts, static_cast<float*>(out.data_ptr()), status, st);
+                              (size_t)ws.numel() - perm - offs - counts, static_cast<float*>(out.data_ptr()), status, st));
   if (rc) return raise(rc);
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -373,10 +388,11 @@ PyObject* moe_block(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   int32_t* ip = static_cast<int32_t*>(idx.data_ptr());
   float* wp = static_cast<float*>(w.data_ptr());
   const cachalot_stream_t st = current_stream(dev);
-  int rc = lib.cachalot_router_logits(x->data_ptr(), gate->data_ptr(), gate_bf16 ? CACHALOT_BF16 : CACHALOT_F32, 1, (int)e, (int)h, logits, st);
+  int rc = UNLOCKED(lib.cachalot_router_logits(x->data_ptr(), gate->data_ptr(), gate_bf16 ? CACHALOT_BF16 : CACHALOT_F32, 1, (int)e, (int)h,
+                                               logits, st));
   if (!rc && want_scores)
-    rc = lib.cachalot_route_topk(logits, c.bias, nullptr, 0, 1, (int)e, c.topk, c.mode, (float)c.temp, (float)c.scale, c.norm, 0, ip, wp, nullptr,
-                             static_cast<float*>(sc.data_ptr()), st);
+    rc = UNLOCKED(lib.cachalot_route_topk(logits, c.bias, nullptr, 0, 1, (int)e, c.topk, c.mode, (float)c.temp, (float)c.scale, c.norm, 0,
+                                          ip, wp, nullptr, static_cast<float*>(sc.data_ptr()), st));
   if (!rc) rc = run_layer(c, x->data_ptr(), logits, routed, ip, wp, dev);
   if (!rc) rc = run_shared(x->data_ptr(), 1, m, c.limit, routed, out.data_ptr(), dev);
   if (rc) return raise(rc);

@@ -94,3 +94,38 @@ def test_block(bank, rule, fused13):
     assert torch.equal(a, b) and torch.equal(ra.indices, rb.indices) and torch.equal(ra.weights, rb.weights) and torch.equal(ra.scores, rb.scores)
     y = cb.shared_expert_forward_batched(_x(5, h), w1=w1, w1_scales=s1, w3=w3, w3_scales=s3, w2=w2, w2_scales=s2)
     assert torch.equal(y, cb.shared_expert_forward_batched(_x(5, h).float(), w1=w1, w1_scales=s1, w3=w3, w3_scales=s3, w2=w2, w2_scales=s2))
+
+
+def test_other_threads_run_while_a_call_waits_for_the_gpu():
+    """A 2-bit batch with bf16 scales is one launch per token: thousands of them fill the launch queue, and the call waits
+    there.  The interpreter's lock is not held meanwhile."""
+    import threading
+    import time
+
+    import cachalot_b200 as cb
+
+    bank = cb.SlabBank(cb.affine_format(2048, 768, 2, 128, "bfloat16"), 2048, 768, 4)
+    bank.fill_random(torch.Generator(device="cuda").manual_seed(1))
+    rows = 6000
+    x, slots, w = _x(rows, 2048), torch.zeros((rows, 2), dtype=torch.int32, device="cuda"), torch.rand((rows, 2), device="cuda")
+    cb.moe_forward(x[:4], slots[:4], w[:4], bank)
+    torch.cuda.synchronize()
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.0005)
+
+    th = threading.Thread(target=tick)
+    th.start()
+    try:
+        t0 = time.perf_counter()
+        out = cb.ops._host.moe_forward(x, slots, w, bank.slab, cb.ops.addressof(bank.desc), 10.0, bank.default_numerics, cb.ops._ODT[torch.float32], None)
+        t1 = time.perf_counter()
+    finally:
+        stop.set()
+        th.join()
+    torch.cuda.synchronize()
+    assert out is not None and t1 - t0 > 0.02, f"the call returned after {t1 - t0:.4f} s: too short to say anything"
+    assert sum(t0 + 0.005 < t < t1 - 0.005 for t in ticks) >= 3
