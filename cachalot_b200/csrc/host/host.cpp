@@ -114,10 +114,11 @@ int unlocked(F&& launch) {
 struct Args {
   PyObject* const* a;
   bool bad = false;
-  long i(int n) {
+  int i(int n) {
     const long v = PyLong_AsLong(a[n]);
     if (v == -1 && PyErr_Occurred()) PyErr_Clear(), bad = true;
-    return v;
+    if (v != (int)v) bad = true;
+    return (int)v;
   }
   double f(int n) {
     const double v = PyFloat_AsDouble(a[n]);
