@@ -1,6 +1,6 @@
 """GPU parity of the grouped f16 tensor-core kernels (several tokens over a 2-bit bank) against the float64 oracle: rows that
-start in mid-group, group 64, tiles and stages that end early, units of 1, 64 and 65 rows, absent experts, more routed rows
-than one plan takes."""
+start in mid-group, group 64, tiles and stages that end early, units of 1 to 64 rows and experts of 65 and more, absent
+experts, more routed rows than one plan takes; and which calls go there instead of token by token."""
 import numpy as np
 import pytest
 
@@ -37,7 +37,7 @@ def _want(x, slots, w, experts, group):
 
 
 @pytest.mark.parametrize("hidden,inter,group", [(128, 64, 64), (256, 192, 128), (512, 320, 64), (1088, 448, 128), (640, 2880, 128)])
-@pytest.mark.parametrize("tokens", [2, 17, 66])
+@pytest.mark.parametrize("tokens", [6, 17, 66])  # six: the fewest that go to these kernels at all five shapes
 def test_batch(hidden, inter, group, tokens):
     import torch
 
@@ -60,10 +60,11 @@ def test_batch(hidden, inter, group, tokens):
     assert torch.equal(cb.moe_forward(*args, out_dtype=torch.bfloat16), got.to(torch.bfloat16))
 
 
-@pytest.mark.parametrize("hidden,inter,group", [(3136, 2880, 64), (3136, 2880, 128), (576, 320, 64)])
+@pytest.mark.parametrize("hidden,inter,group", [(3136, 2880, 64), (3136, 2880, 128), (576, 320, 64), (4096, 2880, 128),
+                                               (5120, 2304, 128), (4096, 2304, 64)])
 def test_stages_with_one_operand_slot(hidden, inter, group):
-    """K of 4i+1 steps of 64 codes, two to four shared-memory stages, several units per CTA: stages that only half of the
-    unpacking warps work on are filled again only when the other half has passed them too."""
+    """K of 4i+1 steps of 64 codes and the sizes of whole banks, two to five shared-memory stages, several units per CTA: stages
+    that only half of the unpacking warps work on are filled again only when the other half has passed them too."""
     import torch
 
     import cachalot_b200 as cb
@@ -170,7 +171,65 @@ def test_more_rows_than_one_plan():
     assert within_bf16_flips(got, _want(x, slots, w, experts, 128))
 
 
-@pytest.mark.parametrize("tokens", [3, 200])
+@pytest.mark.parametrize("hidden,inter,group", [(256, 192, 128), (1088, 448, 64)])
+def test_units(hidden, inter, group):
+    """Experts of 1, 16, 17, 63, 64, 65 and 129 rows: units that end at, before and behind the sixteens of a tile's loads, and
+    one, two and three units of an expert."""
+    import torch
+
+    import cachalot_b200 as cb
+
+    rng = np.random.default_rng(group)
+    counts = [1, 16, 17, 63, 64, 65, 129]
+    experts, bank = _bank(rng, hidden, inter, len(counts), group)
+    slots = rng.permutation(np.repeat(np.arange(len(counts), dtype=np.int32), counts))[:, None]
+    x = configs.round_bf16(rng.standard_normal((len(slots), hidden)).astype(np.float32))
+    w = rng.uniform(0.1, 1.0, slots.shape).astype(np.float32)
+    got = cb.moe_forward(bf16_tensor(x), torch.from_numpy(slots).cuda(), torch.from_numpy(w).cuda(), bank).cpu().numpy()
+    want = _want(x, slots, w, experts, group)
+    for e in range(len(counts)):
+        mine = slots[:, 0] == e
+        assert within_bf16_flips(got[mine], want[mine]), f"expert of {counts[e]} rows"
+
+
+@pytest.mark.parametrize("scale_dtype,small", [("bfloat16", False), ("float16", True)])
+def test_token_by_token_where_the_kernels_do_not_apply(scale_dtype, small):
+    """A bank with bf16 scales, and a chunk that gets only the scratch of the token-by-token route (what a caller that sized it
+    before the grouped kernels came hands over): the bits of one call per token."""
+    import ctypes
+
+    import torch
+
+    import cachalot_b200 as cb
+    from cachalot_b200 import _lib
+
+    hidden, inter, k, tokens, n = 1024, 512, 3, 40, 8
+    g = torch.Generator(device="cuda").manual_seed(5)
+    bank = cb.SlabBank(cb.affine_format(hidden, inter, 2, 128, scale_dtype), hidden, inter, n, layers=1, n_experts=n)
+    bank.fill_random(g)
+    x = torch.randn((tokens, hidden), device="cuda", generator=g).to(torch.bfloat16)
+    ids = torch.rand((tokens, n), device="cuda", generator=g).topk(k, 1).indices.to(torch.int32)
+    w = torch.rand((tokens, k), device="cuda", generator=g) + 0.1
+    one = torch.cat([cb.moe_forward(x[i:i + 1], ids[i:i + 1], w[i:i + 1], bank) for i in range(tokens)])
+    if not small:
+        assert torch.equal(cb.moe_forward(x, ids, w, bank), one)
+        assert torch.equal(cb.moe_prefill_grouped(x, ids, w, bank), one)
+        return
+    assert not torch.equal(cb.moe_prefill_grouped(x, ids, w, bank), one)  # with room it takes the grouped kernels
+    up = lambda v: -(-v // 256) * 256  # noqa: E731
+    need = up(tokens * k * inter * 4) + up(tokens * k * 4)
+    perm, offsets = cb.group_rows(ids, n)
+    out, status = torch.zeros((tokens, hidden), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ws = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
+    call = lambda size: _lib.lib.cachalot_moe_prefill(  # noqa: E731
+        bank.slab.data_ptr(), ctypes.byref(bank.desc), x.data_ptr(), perm.data_ptr(), offsets.data_ptr(), bank.slot_table[0].data_ptr(),
+        w.data_ptr(), tokens, k, n, 10.0, 0, up(ws.data_ptr()), size, out.data_ptr(), status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert call(need - 1) == _lib.ESCRATCH
+    assert call(need) == _lib.OK
+    assert torch.equal(out, one) and int(status.item()) == 0
+
+
+@pytest.mark.parametrize("tokens", [5, 200])
 def test_prefill(tokens):
     import torch
 
