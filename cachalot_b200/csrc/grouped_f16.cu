@@ -22,8 +22,8 @@
 // codes); the MMAs of a unit of 64 rows take 128.  So the unpacked operand goes registers -> TMEM (tcgen05.st, 32 cycles a
 // tile), not through shared memory, where writing and reading it again would take 256 cycles.  Sixteen warps unpack, four
 // per scheduler: a tile's step takes 455 to 476 cycles in a loop of eight warps by themselves, and sixteen instead of
-// eight took 2048 tokens from 4.85 to 4.28 ms.  In the kernel (64 experts, 3072 rows, gate/up) the schedulers issue in 66 %
-// of the cycles, 1200 instructions per tile with scales, waits and addresses: issue slots bound it, not DRAM (16 %).
+// eight took 2048 tokens from 4.85 to 4.28 ms.  In the kernel (64 experts, 3072 rows, gate/up) the schedulers issue in 65 %
+// of the cycles, 1080 instructions per tile with scales, waits and addresses: issue slots bound it, not DRAM (18 %).
 //
 // Warp roles (768 threads): warp 0 TMA (weight tiles through a 3-D map {K/4 bytes, rows, slot}, activation rows
 // sixteen at a time), warp 1 owns TMEM and issues the MMAs, warps 4-19 unpack (four per TMEM lane quarter),
@@ -41,7 +41,6 @@ constexpr int X_PIECE = NT * 128;  // 64 fp16 of every row
 constexpr int X_BOX = 16 * 128;    // one TMA box: 16 rows
 constexpr int NTHREADS = 768;
 constexpr int UNPACK0 = 4, DRAIN0 = 20;  // first unpacking and draining warp
-constexpr int N_UNPACK = DRAIN0 - UNPACK0;
 constexpr int TMEM_COLS = 512;
 constexpr int A_COL = 256;        // operand slots start behind the accumulators
 constexpr int MAX_STAGES = 5, BAR_BYTES = 512;
@@ -144,10 +143,8 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    // A stage is free when its last MMA is done and every unpacking warp has passed it.  The MMAs alone do not say that:
-    // a stage with one operand slot waits for the eight warps of one set only, and a warp of the other set that came to
-    // full[s] after the next fill would take that phase for the one before its own and wait for good.
-    for (int s = 0; s < n_stage; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1 + N_UNPACK);
+    // a stage is free when its last MMA is done: the unpacking warps that wait for the stage have read it before that
+    for (int s = 0; s < n_stage; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1);
     for (int s = 0; s < A_SLOTS; ++s) mbar_init(&a_full[s], 8), mbar_init(&a_empty[s], 1);
     for (int b = 0; b < 2; ++b) mbar_init(&acc_full[b], 1), mbar_init(&acc_empty[b], 4);
     for (int b = 0; b < 8; ++b) mbar_init(&sc_full[b], 2);
@@ -342,17 +339,16 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
       if (!__all_sync(0xffffffffu, mbar_wait(&sc_full[p * 4 + q], par, abort))) break;  // both warps: arrived, and done with the other buffer
       par ^= 1;
       if (w + gridDim.x < total) nxt = fetch(w + gridDim.x, par);
-      for (int ks = 0; ks < n_st && ok; ++ks) {
-        const int steps = steps_of(ks);
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort))) { ok = false; break; }
+      auto stage = [&](int ks, int steps, bool codes) -> bool {
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort))) return false;
         const uint32_t row = smem_u32(smem) + s * STAGE_BYTES + (NA == 2 ? p * W_TILE : 0) + m * (KST / 4);
         for (int i = 0; i < steps; i += (NA == 2 ? 1 : 2), next_slot()) {
           if ((a & 1) != hh) continue;
           const int step = NA == 2 ? i : i + p;
-          if (!begin()) { ok = false; break; }
+          if (!begin()) return false;
           if (step < steps) {
             uint32_t r[32];
-            if (ks < n_main) {
+            if (codes) {
               uint4 wv;
               asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                            : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
@@ -368,9 +364,23 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
           }
           publish();
         }
-        if (!ok) break;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);
+        return true;
+      };
+      // Full stages of codes in a loop of their own (2048 tokens 4.27 -> 3.96 ms: four steps known to the compiler).
+      int ks = 0;
+      for (; ks < n64 / 4 && ok; ++ks) {
+        ok = stage(ks, 4, true);
+        if (++s == n_stage) s = 0, ph ^= 1u;
+      }
+      // A set of warps waits for the stages that it unpacks a slot of, and for no other: the MMAs that free a stage do not
+      // wait for it there, so it could come after the stage's next fill, take that phase for the one before its own and
+      // wait for good.  A phase that it did not wait for is over when it comes to that stage again: stages with one slot
+      // are among the last n_ext + 1 of an item, at most n_stage (enough_stages), and between two items it meets
+      // (sc_full) the warp of the other set that did wait.
+      for (; ks < n_st && ok; ++ks) {
+        const int steps = steps_of(ks);
+        if (steps > (NA == 2 ? 1 : 2) || (a & 1) == hh) ok = stage(ks, steps, ks < n_main);
+        else next_slot();
         if (++s == n_stage) s = 0, ph ^= 1u;
       }
     }
@@ -502,12 +512,15 @@ int windows(int k, int group) {
   return (2 * g + (aligned ? 0 : 14) + 15) / 16;
 }
 size_t scale_bytes(int n_win) { return (size_t)8 * n_win * BM * 16; }  // [buffer][set][scale, bias][window][row]
-// as many stages as fit beside the scales; below two there is no pipeline
+// as many stages as fit beside the scales
 int stages(int na, int n_win) {
   const size_t fixed = scale_bytes(n_win) + BAR_BYTES + 1024;
   if (fixed >= SMEM_LIMIT) return 0;
   return (int)min((SMEM_LIMIT - fixed) / (size_t)(na * W_TILE + (KST / 64) * X_PIECE), (size_t)MAX_STAGES);
 }
+// enough stages: two for a pipeline, and those at the end of an item that may have one operand slot only, the group sums'
+// and the last one of the codes, in different ones
+bool enough_stages(int na, int k, int group) { return stages(na, windows(k, group)) >= 1 + (k_shape(k, group).ext / 64 + 1) / 2; }
 size_t smem_bytes(int na, int nstage, int n_win) {
   return (size_t)nstage * (na * W_TILE + (KST / 64) * X_PIECE) + scale_bytes(n_win) + BAR_BYTES + 1024;
 }
@@ -597,8 +610,8 @@ int run_f16(const BankView& v, const F16Scratch& s, const void* x_bf16, long lon
 }  // namespace
 
 bool f16_supported(const BankView& v) {
-  return v.format == CACHALOT_BANK_AFFINE && v.bits == 2 && v.scale_dtype == CACHALOT_F16 && stages(2, windows(v.hidden, v.group)) >= 2 &&
-         stages(1, windows(v.inter, v.group)) >= 2;
+  return v.format == CACHALOT_BANK_AFFINE && v.bits == 2 && v.scale_dtype == CACHALOT_F16 && enough_stages(2, v.hidden, v.group) &&
+         enough_stages(1, v.inter, v.group);
 }
 
 // as few runs of whole tokens as the planning kernel's limit allows, as equal as they can be

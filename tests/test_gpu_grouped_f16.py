@@ -86,7 +86,7 @@ def test_stages_with_one_operand_slot(hidden, inter, group):
 
 
 @pytest.mark.parametrize("general", [False, True])
-@pytest.mark.parametrize("tokens,experts,grouped", [(64, 128, False), (512, 128, True)])
+@pytest.mark.parametrize("tokens,experts,grouped", [(32, 128, False), (512, 128, True)])
 def test_prefill_scratch(tokens, experts, grouped, general):
     """A chunk that goes token by token takes the scratch of that route only; a grouped one two buffers of 16-bit rows."""
     import torch
@@ -102,13 +102,14 @@ def test_prefill_scratch(tokens, experts, grouped, general):
     args = (x.float() if general else x, ids, w, bank)
     cb.ops._workspaces.clear()
     torch.cuda.synchronize()
-    before = torch.cuda.memory_allocated()
     torch.cuda.reset_peak_memory_stats()
+    # bytes asked for: a block that the allocator hands out again may be up to 1 MiB larger than the request
+    before = torch.cuda.memory_stats()["requested_bytes.all.current"]
     out = cb.moe_prefill_grouped(*args)
-    used = torch.cuda.max_memory_allocated() - before - out.numel() * 4 - (x.numel() * 2 if general else 0)
+    used = torch.cuda.memory_stats()["requested_bytes.all.peak"] - before - out.numel() * 4 - (x.numel() * 2 if general else 0)
     rows = tokens * k
     need = rows * 2 * (hidden + 128 + hidden) if grouped else rows * inter * 4
-    assert used <= need + rows * 64 + (2 << 20), f"{used} bytes for {rows} rows"
+    assert used <= need + rows * 64 + (1 << 18), f"{used} bytes for {rows} rows"  # + per-row plans, per-expert counts
 
 
 def test_infinite_and_nan_activations():
