@@ -1,14 +1,15 @@
 // Routed experts of several tokens over the 2-bit affine bank on the f16 tensor cores (tcgen05.mma kind::f16, weights
 // as the TMEM operand).
 //
-// A weight is s*q + b with one fp16 pair (s, b) per group of 64 or 128 codes q in 0..3.  Written as
+// A weight is s*q + b with one fp16 pair (s, b) per group of 128 codes q in 0..3.  Written as
 // s*(q-1) + (b+s), the first term is one of {-s, 0, s, 2s}: exact in fp16 (up to |s| = 32752), so the MMA multiplies
 // the true weight and no scale has to be applied to partial sums.  The second term only needs the sums of the
 // activations over the groups; they enter the same accumulator as further K columns: [b | s] against the group sums
 // split into two fp16 halves (22 bits).  Activations are bf16, so after scaling a row by a power of two (its largest
 // value into [2^7, 2^8)) they are exact in fp16 down to 2^-25 of the row's largest value.  Against float64 with the same
 // bf16 roundings a call is off by 1e-4 to 1.8e-4 of its norm (values that rounded the other way), the one-token kernel,
-// which holds activations in fixed point, by 2.1e-4 to 2.7e-4, the one-warp kernels for groups of 64 by 1.3e-5.
+// whose place it takes and which holds activations in fixed point, by 2.1e-4 to 2.7e-4.  The one-warp kernels, at 1.3e-5
+// with groups of 64, keep the banks that the one-token kernel does not take.
 //
 // Rows are grouped by expert.  Two grouped GEMMs run per call, weights on the M side:
 //   gate/up : [128 weight rows, <=64 routed rows] twice, K = hidden; g, u rounded to bf16, SwiGLU, router weight,
@@ -70,10 +71,10 @@ __device__ __forceinline__ uint32_t idesc_f16(int n) { return (1u << 4) | ((uint
 struct KShape {
   int k, block, n_block, ext, pitch;
 };
-__host__ __device__ inline KShape k_shape(int k, int group) {
+__host__ __device__ inline KShape k_shape(int k) {
   KShape s;
   s.k = k;
-  s.block = (group == 128 && k % 128 == 0) ? 128 : 64;  // rows that start in mid-group: half groups
+  s.block = k % 128 == 0 ? 128 : 64;  // rows that start in mid-group: half groups
   s.n_block = k / s.block;
   s.ext = (2 * s.n_block + 63) / 64 * 64;
   s.pitch = k + 2 * s.ext;
@@ -84,7 +85,6 @@ struct F16Args {
   const uint8_t* bank;
   long long record_bytes;
   long long off_s[2], off_b[2];  // scale and bias arrays of the matrices inside a record
-  int group;
   const Unit* units;
   const int32_t* n_units;
   int n_rows, k;
@@ -163,7 +163,7 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
 
   const int n_mt = (A.n_rows + BM - 1) / BM;
   const long long total = (long long)*A.n_units * n_mt;
-  const KShape K = k_shape(A.k, A.group);
+  const KShape K = k_shape(A.k);
   const int n64 = A.k / 64, n_main = (n64 + 3) / 4;         // 64-code steps; stages of four
   const int e64 = K.ext / 64, n_ext = (e64 + 1) / 2;        // group-sum steps; stages of two (each: high and low half)
   const int n_st = n_main + n_ext;
@@ -258,7 +258,6 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
     // TMEM lane quarter; matrix (gate/up) or step of a slot (down); which of every two operand slots
     const int q = warp & 3, p = ((warp - UNPACK0) >> 2) & 1, hh = (warp - UNPACK0) >> 3;
     const int m = q * 32 + lane;                  // row of the tile
-    const int sh = A.group == 128 ? 1 : 0;        // groups per 64 codes: one or a half
     const uint32_t t_dst = tmem + A_COL + ((uint32_t)(q * 32) << 16) + p * 32;
     // The scales and biases of the next item come by 16-byte asynchronous copies (a row of them starts at any even
     // address) into windows [buffer][set][array][window][row].  The two warps that unpack the same rows (hh) share them:
@@ -279,7 +278,7 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
       r.i0 = n * n64;
       const uint32_t dst = smem_u32(sc_base) + (uint32_t)((par * 2 + p) * 2 * A.n_win * BM + m) * 16;
       r.buf = dst;
-      const long long g0 = r.i0 >> sh, g1 = (r.i0 + n64 - 1) >> sh;
+      const long long g0 = r.i0 >> 1, g1 = (r.i0 + n64 - 1) >> 1;  // two steps of 64 codes to a group
 #pragma unroll
       for (int arr = 0; arr < 2; ++arr) {
         const uintptr_t at = reinterpret_cast<uintptr_t>(rec + (arr ? off_b : off_s) + 2 * g0);
@@ -302,13 +301,11 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
       asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(r.buf + (uint32_t)((arr * A.n_win + (h >> 3)) * BM * 16 + (h & 7) * 2)));
       return v;
     };
-    const int blk_sh = (A.group == 128 && K.block == 64) ? 1 : 0;
-    const int blk_per = K.block / 64;  // 64-code steps per block
     auto ext_val = [&](const RowRef& r, int e) -> uint32_t {
       if (!r.ok || e >= 2 * K.n_block) return 0u;
       const bool is_s = e >= K.n_block;
       const int j = is_s ? e - K.n_block : e;
-      return value(r, is_s ? 0 : 1, blk_per == 2 ? j : ((r.i0 + j) >> blk_sh) - (r.i0 >> blk_sh));
+      return value(r, is_s ? 0 : 1, K.block == 128 ? j : ((r.i0 + j) >> 1) - (r.i0 >> 1));
     };
     int s = 0, a = 0;
     uint32_t ph = 0, aph = 1;  // the first pass over the slots finds them free
@@ -353,7 +350,7 @@ grouped_f16_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_cons
               asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                            : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
                            : "r"(row + ((step ^ ((m >> 1) & 3)) << 4)));
-              const uint32_t sv = cur.ok ? value(cur, 0, ((cur.i0 + ks * 4 + step) >> sh) - (cur.i0 >> sh)) : 0u;
+              const uint32_t sv = cur.ok ? value(cur, 0, ((cur.i0 + ks * 4 + step) >> 1) - (cur.i0 >> 1)) : 0u;
               unpack64(wv, sv * 0x10001u, r);
             } else {
               const int e0 = ((ks - n_main) * 2 + step) * 64;
@@ -506,9 +503,9 @@ __global__ void prep_rows_kernel(const __nv_bfloat16* __restrict__ x, const int3
 
 constexpr size_t SMEM_LIMIT = 227 * 1024;
 // windows of a row of scales: its halfs behind up to 14 bytes of lead-in, none where every row starts on 16 bytes
-int windows(int k, int group) {
-  const int g = (k + group - 1) / group + (k % group ? 1 : 0);
-  const bool aligned = k % group == 0 && (k / group) % 8 == 0;
+int windows(int k) {
+  const int g = (k + 127) / 128 + (k % 128 ? 1 : 0);
+  const bool aligned = k % 1024 == 0;
   return (2 * g + (aligned ? 0 : 14) + 15) / 16;
 }
 size_t scale_bytes(int n_win) { return (size_t)8 * n_win * BM * 16; }  // [buffer][set][scale, bias][window][row]
@@ -520,7 +517,7 @@ int stages(int na, int n_win) {
 }
 // enough stages: two for a pipeline, and those at the end of an item that may have one operand slot only, the group sums'
 // and the last one of the codes, in different ones
-bool enough_stages(int na, int k, int group) { return stages(na, windows(k, group)) >= 1 + (k_shape(k, group).ext / 64 + 1) / 2; }
+bool enough_stages(int na, int k) { return stages(na, windows(k)) >= 1 + (k_shape(k).ext / 64 + 1) / 2; }
 size_t smem_bytes(int na, int nstage, int n_win) {
   return (size_t)nstage * (na * W_TILE + (KST / 64) * X_PIECE) + scale_bytes(n_win) + BAR_BYTES + 1024;
 }
@@ -553,7 +550,7 @@ F16Scratch carve_f16(uint8_t* base, const BankView& v, size_t R, size_t n_seg) {
   s.x_scale = reinterpret_cast<float*>(take(R * 4));
   s.h_scale = reinterpret_cast<float*>(take(R * 4));
   // x is through when h is prepared, and h when y is written: two buffers serve the four
-  s.xp = s.hp = reinterpret_cast<__half*>(take(R * max(k_shape(v.hidden, v.group).pitch, k_shape(v.inter, v.group).pitch) * 2));
+  s.xp = s.hp = reinterpret_cast<__half*>(take(R * max(k_shape(v.hidden).pitch, k_shape(v.inter).pitch) * 2));
   s.h = s.y = reinterpret_cast<__nv_bfloat16*>(take(R * max(v.hidden, v.inter) * 2));
   s.total = at;
   return s;
@@ -562,7 +559,7 @@ F16Scratch carve_f16(uint8_t* base, const BankView& v, size_t R, size_t n_seg) {
 // planned rows -> s.y
 int run_f16(const BankView& v, const F16Scratch& s, const void* x_bf16, long long R, float limit, int* status, cudaStream_t stream) {
   const int H = v.hidden, I = v.inter;
-  const KShape kx = k_shape(H, v.group), kh = k_shape(I, v.group);
+  const KShape kx = k_shape(H), kh = k_shape(I);
   CUtensorMap m_w1, m_w3, m_w2, m_x, m_h;
   int rc;
   if ((rc = make_map(&m_w1, v.base + v.off[0], H / 4, H / 4, I, v.record_bytes, v.n_slots, BM, KST / 4))) return rc;
@@ -576,7 +573,6 @@ int run_f16(const BankView& v, const F16Scratch& s, const void* x_bf16, long lon
   F16Args a = {};
   a.bank = v.base;
   a.record_bytes = v.record_bytes;
-  a.group = v.group;
   a.units = s.plan.units;
   a.n_units = s.plan.n_units;
   a.row_w = s.plan.row_w;
@@ -590,7 +586,7 @@ int run_f16(const BankView& v, const F16Scratch& s, const void* x_bf16, long lon
   a.row_scale = s.x_scale;
   a.out = s.h;
   auto launch = [&](auto kern, int na, const CUtensorMap& ma0, const CUtensorMap& ma1, const CUtensorMap& mb) {
-    a.n_win = windows(a.k, a.group);
+    a.n_win = windows(a.k);
     a.n_stage = stages(na, a.n_win);
     smem_optin_once(kern, (int)SMEM_LIMIT);
     kern<<<sms, NTHREADS, smem_bytes(na, a.n_stage, a.n_win), stream>>>(ma0, ma1, mb, a);
@@ -610,8 +606,8 @@ int run_f16(const BankView& v, const F16Scratch& s, const void* x_bf16, long lon
 }  // namespace
 
 bool f16_supported(const BankView& v) {
-  return v.format == CACHALOT_BANK_AFFINE && v.bits == 2 && v.scale_dtype == CACHALOT_F16 && enough_stages(2, v.hidden, v.group) &&
-         enough_stages(1, v.inter, v.group);
+  return v.format == CACHALOT_BANK_AFFINE && v.bits == 2 && v.group == 128 && v.scale_dtype == CACHALOT_F16 && enough_stages(2, v.hidden) &&
+         enough_stages(1, v.inter);
 }
 
 // as few runs of whole tokens as the planning kernel's limit allows, as equal as they can be

@@ -286,7 +286,7 @@ static int grouped_tc_min_rows() {  // CACHALOT_GROUPED_MIN_ROWS overrides the b
   return v;
 }
 #define GROUPED_TC_MIN_ROWS grouped_tc_min_rows()
-// 2-bit bank with fp16 scales, reference rounding points: do the grouped f16 kernels beat the one-token kernel?  Both sides
+// 2-bit bank with fp16 scales and groups of 128, reference rounding points: do the grouped f16 kernels beat the one-token kernel?  Both sides
 // in us, fitted to 480 timings (2048 x 768 to 5120 x 2304, 1 to 384 experts, 3 to 1024 routed rows of one or six per token,
 // uniform and Zipf routing).  The grouped kernels take 30 + 5.5 per 1000 of hidden + inter for their launches and one
 // unit's walk over K, and unpack every unit of up to 64 rows of one expert: 0.4 + 0.68 per million weights of a matrix.
@@ -307,9 +307,14 @@ static BankView shape_view(const cachalot_bank_desc* d) {
   return v;
 }
 
+// The grouped kernels take the place of the one-token kernel only.  They are nearer to float64 than that one; the one-warp
+// kernels, which run where it does not (groups of 64, more than eight experts per token, hidden sizes off 128), are nearer
+// still and keep those calls.
+static bool f16_replaces(const BankView& v, int k) { return f16_supported(v) && decode_fused_supported(v, 1, k); }
+
 // a batch goes in runs of equal length, each of which unpacks its experts anew: the rule is asked for one of them
 static bool decode_f16_takes(const BankView& v, int rows, int k, int n_slots) {
-  return f16_supported(v) && grouped_f16_pays(v, decode_f16_run(rows, k), k, n_slots);
+  return f16_replaces(v, k) && grouped_f16_pays(v, decode_f16_run(rows, k), k, n_slots);
 }
 
 // what moe_decode cannot do without; with less than cachalot_moe_decode_workspace_bytes a 2-bit bank goes token by token
@@ -327,7 +332,7 @@ extern "C" size_t cachalot_moe_decode_workspace_bytes(const cachalot_bank_desc* 
   if (!desc || rows <= 0 || k <= 0) return 0;
   const size_t m = decode_min_workspace(desc, rows, k);
   const BankView v = shape_view(desc);
-  const size_t f = k <= 64 && decode_f16_takes(v, rows, k, desc->n_slots) ? decode_f16_workspace_bytes(v, rows, k) : 0;
+  const size_t f = decode_f16_takes(v, rows, k, desc->n_slots) ? decode_f16_workspace_bytes(v, rows, k) : 0;
   return m > f ? m : f;
 }
 
@@ -506,7 +511,7 @@ static size_t prefill_min_workspace(const cachalot_bank_desc* desc, int tokens, 
 }
 
 static bool prefill_f16_takes(const BankView& v, int tokens, int k, int n_experts, int mxfp4_act) {
-  return !mxfp4_act && f16_supported(v) && n_experts <= 8192 && grouped_f16_pays(v, tokens, k, n_experts);
+  return !mxfp4_act && f16_replaces(v, k) && n_experts <= 8192 && grouped_f16_pays(v, tokens, k, n_experts);
 }
 
 extern "C" size_t cachalot_moe_prefill_workspace_bytes(const cachalot_bank_desc* desc, int tokens, int k, int mxfp4_act) {
