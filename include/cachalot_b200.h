@@ -156,7 +156,8 @@ CACHALOT_API size_t cachalot_moe_decode_workspace_bytes(const cachalot_bank_desc
  * clamp skipped when swiglu_limit <= 0, and a slot < 0 contributing zeros
  * (minimax/gpu_select.py:265-273).  x bf16 [rows,H]; slots i32 [rows,k]; gate_w f32 [rows,k];
  * out f32 [rows,H] (or bf16 when out_dtype == CACHALOT_BF16).  The reference runs one token at a
- * time (model/moe_layer_metal.py:168-171); rows > 1 is the same math per row. */
+ * time (model/moe_layer_metal.py:168-171); rows > 1 is the same math per row.  Several tokens over a 2-bit bank with fp16
+ * scales may run on kernels that hold scale * (code - 1) in fp16: scales up to 32752 in magnitude there. */
 CACHALOT_API int cachalot_moe_decode(const void* bank, const cachalot_bank_desc* desc /* host */, const void* x_bf16,
                         const int32_t* slots, const float* gate_w, int rows, int k, float swiglu_limit,
                         int numerics, void* workspace, size_t workspace_bytes, void* out, int out_dtype,
